@@ -176,6 +176,27 @@ def test_gemm_f32_rows_do_not_depend_on_batch(k):
         assert torch.equal(one[0], full[row])
 
 
+@pytest.mark.parametrize("N,K,offset", [(129, 300, 0), (2048, 1536, 0), (16500, 68, 0), (200, 2050, 0), (129, 512, 1)])
+def test_gemm_f32_every_tile_sums_alike(k, N, K, offset):
+    """Steps of any number of rows, weights with one range of K and with eight, inner sizes that 16-byte
+    copies cannot take and an operand off their boundary: a row has the same bits whatever tile made it."""
+    gen = torch.Generator().manual_seed(N + K)
+    store = torch.randn(260 * K + offset, generator=gen).cuda()
+    a = store[offset:].view(260, K)
+    w, b = torch.randn(N, K, generator=gen).cuda(), torch.randn(N, generator=gen).cuda()
+    one = torch.empty(260, N, device="cuda")
+    for row in range(0, 260, 4):
+        k.gemm_f32(a[row : row + 4], w, b, one[row : row + 4], 4)
+    want = a.double() @ w.double().T + b.double()
+    # As in test_gemm_f32.
+    assert (one.double() - want).abs().max().item() <= 2 * 2.0 ** -24 * math.sqrt(K) * want.abs().max().item() + 1e-6
+    for M in (1, 2, 5, 8, 9, 16, 17, 24, 40, 41, 64, 75, 80, 81, 112, 153, 260):
+        out = torch.full((M + 1, N), 5.0, device="cuda")
+        k.gemm_f32(a, w, b, out, M)
+        assert torch.equal(out[:M], one[:M]), M
+        assert torch.all(out[M] == 5.0)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,T", [(1536, 700), (3584, 300), (240, 513), (4100, 260)])
 def test_add_rmsnorm_many_rows(k, dtype, hidden, T):

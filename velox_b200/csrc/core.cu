@@ -1,6 +1,5 @@
 // Row-wise kernels of the model step: embedding, fused residual-add + RMSNorm, rotate-half RoPE
-// fused with the K/V write into the paged cache, SwiGLU, and a float32 SIMT GEMM for the true
-// 32-bit path.  All arithmetic that the engine promises in 32-bit (norm statistics, rotation,
+// fused with the K/V write into the paged cache, and SwiGLU.  All arithmetic that the engine promises in 32-bit (norm statistics, rotation,
 // the residual sum, SiLU) is float32 here whatever the storage type.
 //
 // Formulas follow the reference engine (paths inside that project):
@@ -412,65 +411,6 @@ __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// float32 GEMM on the FP32 pipes (no tensor cores, no TF32): C[M,N] = A[M,K] * W[N,K]^T + bias.
-// Every output element is summed over k = 0..K-1 in order by one thread, so a row's result does
-// not depend on M or on where the row sits in the batch.
-// ---------------------------------------------------------------------------------------------
-constexpr int GF_BM = 64, GF_BN = 64, GF_BK = 16;
-
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                const float* __restrict__ bias, float* __restrict__ C, int M, int N, int K) {
-  allow_dependents();
-  grid_dependency_wait();
-  __shared__ float As[GF_BK][GF_BM + 4];
-  __shared__ float Ws[GF_BK][GF_BN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * GF_BM, n0 = blockIdx.x * GF_BN;
-  const int ty = tid >> 4, tx = tid & 15;
-  const int load_row = tid >> 2, load_k = (tid & 3) * 4;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-  for (int k0 = 0; k0 < K; k0 += GF_BK) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int k = k0 + load_k + j;
-      const int am = m0 + load_row, wn = n0 + load_row;
-      As[load_k + j][load_row] = (am < M && k < K) ? A[(size_t)am * K + k] : 0.f;
-      Ws[load_k + j][load_row] = (wn < N && k < K) ? W[(size_t)wn * K + k] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < GF_BK; ++k) {
-      float a[4], w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) w[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < N) C[(size_t)m * N + n] = acc[i][j] + (bias ? bias[n] : 0.f);
-    }
-  }
-}
-
 // bf16 -> float32 copy of selected rows (logits of the bfloat16 path are returned as float32).
 __global__ void cast_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ in,
                                         float* __restrict__ out, long long total) {
@@ -819,14 +759,6 @@ VX_API int vx_swiglu(const void* gate_up, void* out, int dtype, int num_tokens, 
   else
     launch_pdl(swiglu_kernel<__nv_bfloat16>, dim3((int)blocks), dim3(threads), 0, stream, 
         (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)out, total, inter);
-  return (int)cudaGetLastError();
-}
-
-VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N,
-                       int K, cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return 0;
-  dim3 grid((N + GF_BN - 1) / GF_BN, (M + GF_BM - 1) / GF_BM);
-  launch_pdl(gemm_f32_kernel, dim3(grid), dim3(256), 0, stream, A, W, bias, C, M, N, K);
   return (int)cudaGetLastError();
 }
 
