@@ -245,7 +245,7 @@ def plain_paged_attention(q, k_all, v_all, ctx, scale, window):
 
 def run_attention_case(k, dtype, H, G, D, P, seqs, window=None, seed=0, min_split_keys=256,
                        target_ctas=296, spike=None, fused_merge=True, max_cluster=1, max_splits=64,
-                       tensor_memory=False, ramp=None, tc_ctas_per_sm=1, tc_merge_us=30.0):
+                       tensor_memory=False, ramp=None, tc_ctas_per_sm=1, tc_merge_us=30.0, spike_scale=12, cache_offset=0):
     """seqs: list of (q_len, ctx_len).  Returns (got, want) as float64 [T, H, D]."""
     from velox_b200.ops import attention_plan as ap
 
@@ -273,9 +273,9 @@ def run_attention_case(k, dtype, H, G, D, P, seqs, window=None, seed=0, min_spli
             page, off = pages[key_index // P], key_index % P
             direction = torch.randn(D, generator=gen)
             direction = direction / direction.norm()
-            k_cache[page, off, :, :] = (direction * 12).to(dtype)
+            k_cache[page, off, :, :] = (direction * spike_scale).to(dtype)
             q_view = qkv[row + qi, : H * D].view(H, D)
-            q_view[:] = (direction * 12).to(dtype)
+            q_view[:] = (direction * spike_scale).to(dtype)
         slots = [pages[i // P] * P + i % P for i in range(kv_len)]
         if ramp is not None:
             # Every query looks along one direction and the keys' share of it grows with the
@@ -306,6 +306,9 @@ def run_attention_case(k, dtype, H, G, D, P, seqs, window=None, seed=0, min_spli
     out = torch.zeros(T, H * D, dtype=dtype, device="cuda")
     partial_o = torch.zeros(max(plan.partial_rows, 1) * D, device="cuda")
     partial_lse = torch.zeros(max(plan.partial_rows, 1), device="cuda")
+    if cache_offset:  # pools that start off a 16-byte boundary
+        k_cache, v_cache = (torch.cat([c.new_zeros(cache_offset), c.flatten()]).cuda()[cache_offset:].view(c.shape)
+                            for c in (k_cache, v_cache))
     args = (qkv.cuda(), out, k_cache.cuda(), v_cache.cuda(), tables.cuda(), dev(q_start), dev(q_lens), dev(kv_lens))
     fused = fused_merge and dtype != torch.float32 and len(plan.merge_items) > 0
     counters = torch.zeros(max(1, len(plan.merge_items) * G), dtype=torch.int32, device="cuda") if fused else None
@@ -397,6 +400,18 @@ def test_attention_cluster_shares_an_item(k, H, G, D, P, max_cluster, max_splits
 
 # One CTA per SM with P in shared memory over the K tile, or two with P in tensor memory.
 TC_FORMS = pytest.mark.parametrize("per_sm", [1, 2], ids=["p_in_shared_memory", "p_in_tensor_memory"])
+
+
+@pytest.mark.parametrize("D,offset", [(16, 0), (48, 0), (128, 0), (128, 1), (256, 0)])
+def test_attention_float32_tiles_at_their_edges(k, D, offset):
+    """One to four warps with rows, one tile of keys and many, last tiles of one key, a range that starts
+    inside a tile, and pools whose rows 16-byte copies cannot take."""
+    seqs = [(1, 0), (1, 31), (1, 32), (3, 64), (5, 60), (33, 130), (2, 511)]
+    for window in (None, 70):
+        got, want, _ = run_attention_case(k, torch.float32, 6, 2, D, 16, seqs, window=window, seed=D, min_split_keys=96,
+                                          target_ctas=200, cache_offset=offset)
+        err = (got - want).abs().max().item()
+        assert err <= _attn_tol(torch.float32) * want.abs().max().item(), (window, err)
 
 
 @TC_FORMS
