@@ -706,6 +706,32 @@ def test_filter_threshold_kernels_agree(k, vocab):
     assert int((logits[8] >= one[8]).sum()) == 1
 
 
+@pytest.mark.parametrize("rows", [18, 19, 36, 37, 64])
+def test_filter_threshold_clusters_of_every_size(k, rows):
+    """Clusters of eight, four and two CTAs a row against one CTA a row, bit for bit: thresholds near the
+    maximum and far from it, bins with more entries than are looked at one by one (ties, a row of equal
+    entries, a narrow row), masked entries and rows off a 16-byte boundary."""
+    gen = torch.Generator().manual_seed(rows)
+    vocab = 50021
+    store = torch.randn(rows, vocab, generator=gen) * (0.01 + 4 * torch.rand(rows, 1, generator=gen))
+    store[0] = 1.5
+    store[1] = store[1].round()  # ties by the thousand
+    store[2] *= 1e-3             # all entries in one bin
+    store[3, 100:] = torch.finfo(torch.float32).min
+    store[4, : vocab - 3] = float("-inf")
+    store[5, 7] = 3e4
+    logits = store.cuda()
+    temps = (0.2 + 1.5 * torch.rand(rows, generator=gen)).cuda()
+    top_k = torch.randint(0, 300, (rows,), generator=gen, dtype=torch.int32).cuda()
+    top_p = torch.tensor([0.5, 0.8, 0.95, 0.999, 1.0])[torch.randint(0, 5, (rows,), generator=gen)].cuda()
+    top_p[0], top_k[0] = 0.4, 0
+    top_p[2], top_k[2] = 0.7, 0
+    one, auto = (torch.full((rows,), 7.0, device="cuda") for _ in range(2))
+    k.filter_threshold(logits, rows, temps, top_k, top_p, one, kind=1)
+    k.filter_threshold(logits, rows, temps, top_k, top_p, auto)
+    assert torch.equal(one.view(torch.int32), auto.view(torch.int32)), (one.tolist(), auto.tolist())
+
+
 def test_filter_threshold_beyond_the_cluster_kernel(k):
     """A row longer than the cluster's registers hold takes the one-CTA kernel; asking for the
     cluster kernel by name is refused."""

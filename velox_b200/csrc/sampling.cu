@@ -169,12 +169,15 @@ sample_kernel(const float* __restrict__ logits, int vocab, long long row_stride,
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = base + j < vocab ? row[base + j] : CUDART_NAN_F;
       }
+      // (Also what lies past the row's end, NaN, is no candidate.)  Behind a filter hardly a group has
+      // one, and the generator's ten rounds are most of what an entry costs.
+      if (!(v[0] * inv_t >= cut || v[1] * inv_t >= cut || v[2] * inv_t >= cut || v[3] * inv_t >= cut)) continue;
       const uint4 bits = philox4x32_10(make_uint4((uint32_t)(base >> 2), draw, 0u, 0u), key);
       const uint32_t b[4] = {bits.x, bits.y, bits.z, bits.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float scaled = v[j] * inv_t;
-        if (!(scaled >= cut)) continue;  // also what lies past the row's end (NaN)
+        if (!(scaled >= cut)) continue;
         const float noise = fmaxf(-logf(uniform_open(b[j])), 1e-10f);
         Best c;
         c.score = scaled - logf(noise);
@@ -461,23 +464,31 @@ filter_threshold_kernel(const float* __restrict__ logits, int vocab, long long r
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same threshold by a cluster of eight CTAs per row, for rows of up to 196,608 entries.  Each
-// CTA reads an eighth of the row once and keeps it in registers (24 entries a thread); what the
-// kernel above does in five sweeps over memory happens here over registers.  Every CTA builds
-// the histogram of its share in its own shared memory and adds the bins that are not empty into
-// the row's histogram, which lies in the shared memory of the cluster's first CTA; that CTA
-// chooses the digit (with the same code as above) and writes it into its peers' shared memory.
-// The normaliser is the sum of the first histogram's masses: all sums are of the same integers
-// as above, so both kernels give the same threshold bit for bit.
+// The same threshold by a cluster of CTAs per row, for rows of up to 196,608 entries.  What bounds it is
+// not the row's bytes (the head has just written them, they are in the L2) but the atomics of entries that
+// share a bin, and the waves of CTAs: so the first histogram is over the distance from the row's maximum,
+// in steps of 1/64, which spreads the entries over hundreds of bins (sign, exponent and two bits of the
+// mantissa put them into a few dozen), and at first it takes only the entries within eight units of the
+// maximum.  The mass of all the others is part of the normaliser, a sum in registers; only when the
+// threshold is not among the near entries are the far ones put into the histogram as well.  The entries of
+// the bin that holds the threshold, a few hundred as a rule, are gathered in the cluster's first CTA, which
+// looks at each: the smallest of them with fewer than k entries and less than top_p of the mass above it.
+// (A threshold is always the value of an entry, since nothing changes between two of them.)  A bin of more
+// than FC_LIST entries is searched digit by digit as in the kernel above.
+//
+// All sums are of the same integers as above and the histogram's bins are in the order of the values, so
+// every form gives the same threshold bit for bit.
 //
 // A 64-bit sum in shared memory is a compare-and-swap loop; the masses (41 bits at most) are
 // therefore added as two 32-bit words, the low word's carry found from the value it held before.
 // ---------------------------------------------------------------------------------------------
-constexpr int FC_CLUSTER = 8;
-constexpr int FC_PER_THREAD = 24;
-constexpr int FC_COPIES = 4;
-constexpr int FC_MAX_VOCAB = FC_CLUSTER * FILTER_THREADS * FC_PER_THREAD;
+constexpr int FC_MAX_VOCAB = 196608;
+constexpr int FC_COPIES = 2;
+constexpr int FC_LIST = 1024;          // entries of the threshold's bin that are looked at one by one
+constexpr float FC_STEPS = 64.0f;      // bins per unit of distance from the maximum
+constexpr int FC_NEAR = 8 * 64;        // bins that the first histogram fills
 constexpr size_t FC_SMEM_BYTES = (size_t)FILTER_BINS * (sizeof(unsigned long long) + sizeof(unsigned int)) +
+                                 (size_t)FC_LIST * (sizeof(unsigned long long) + sizeof(unsigned int)) +
                                  (size_t)FC_COPIES * FILTER_BINS * 3 * sizeof(unsigned int);
 
 __device__ __forceinline__ void add_mass_words(unsigned int* lo, unsigned int* hi, uint32_t bin, unsigned long long w) {
@@ -503,6 +514,13 @@ __device__ __forceinline__ T* cluster_peer(T* local, unsigned int rank) {
   return reinterpret_cast<T*>(out);
 }
 
+// The bin of a value: bin FILTER_BINS - 1 starts at the row's maximum.  Monotone in s, infinities included.
+__device__ __forceinline__ int distance_bin(float s, float top) {
+  const float steps = s == top ? 0.f : fminf((top - s) * FC_STEPS, (float)(FILTER_BINS - 1));
+  return FILTER_BINS - 1 - (int)steps;
+}
+
+template <int CLUSTER>
 __global__ void __launch_bounds__(FILTER_THREADS, 1)
 filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, long long row_stride,
                                 const float* __restrict__ temperature, const int* __restrict__ top_k,
@@ -510,20 +528,23 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
   __shared__ float scratch[32];
   __shared__ unsigned int sc[32];
   __shared__ unsigned long long sm[32];
-  __shared__ float peer_max[FC_CLUSTER];
-  __shared__ unsigned int chosen_digit;
+  __shared__ float peer_max[CLUSTER];
+  __shared__ unsigned long long peer_total[CLUSTER];
+  __shared__ unsigned int chosen_digit, chosen_entries, listed;
   __shared__ DigitChoice choice;
   extern __shared__ __align__(16) unsigned char filter_smem[];
   unsigned long long* row_mass = reinterpret_cast<unsigned long long*>(filter_smem);   // [BINS], used in CTA 0
-  unsigned int* row_count = reinterpret_cast<unsigned int*>(row_mass + FILTER_BINS);    // [BINS], used in CTA 0
-  unsigned int* own_count = row_count + FILTER_BINS;                                    // [COPIES][BINS]
+  unsigned long long* list_mass = row_mass + FILTER_BINS;                               // [LIST], used in CTA 0
+  unsigned int* row_count = reinterpret_cast<unsigned int*>(list_mass + FC_LIST);       // [BINS], used in CTA 0
+  unsigned int* list_key = row_count + FILTER_BINS;                                     // [LIST], used in CTA 0
+  unsigned int* own_count = list_key + FC_LIST;                                         // [COPIES][BINS]
   unsigned int* own_lo = own_count + FC_COPIES * FILTER_BINS;
   unsigned int* own_hi = own_lo + FC_COPIES * FILTER_BINS;
   allow_dependents();
   grid_dependency_wait();
   unsigned int rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  const int r = blockIdx.x / FC_CLUSTER;
+  const int r = blockIdx.x / CLUSTER;
   const int tid = (int)threadIdx.x;
   const float temp = temperature[r];
   const int k = top_k[r];
@@ -535,29 +556,13 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
     if (rank == 0u && tid == 0) threshold[r] = -CUDART_INF_F;
     return;
   }
-  const float* row = logits + (size_t)r * row_stride;
   const float inv_t = 1.0f / fmaxf(temp, 1e-5f);
-  const bool vectors = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  // This CTA's share of the row, a multiple of four entries.
+  const int share = ((vocab + CLUSTER - 1) / CLUSTER + 3) / 4 * 4;
+  const int begin = min(vocab, (int)rank * share), entries = min(vocab, begin + share) - begin;
+  const float* own_row = logits + (size_t)r * row_stride + begin;
+  const bool vectors = (reinterpret_cast<uintptr_t>(own_row) & 15) == 0;
 
-  // This CTA's share in groups of four entries, the threads side by side; what lies past the
-  // share or the row is NaN, which no step below counts.
-  const int groups = (vocab + 3) >> 2;
-  const int share = (groups + FC_CLUSTER - 1) / FC_CLUSTER;
-  const int group_begin = (int)rank * share, group_end = min(groups, group_begin + share);
-  float s[FC_PER_THREAD];
-#pragma unroll
-  for (int j = 0; j < FC_PER_THREAD / 4; ++j) {
-    const int g = group_begin + j * FILTER_THREADS + tid;
-    const int base = g << 2;
-    if (g < group_end && vectors && base + 4 <= vocab) {
-      const float4 q = reinterpret_cast<const float4*>(row)[g];
-      s[4 * j] = __fmul_rn(q.x, inv_t), s[4 * j + 1] = __fmul_rn(q.y, inv_t), s[4 * j + 2] = __fmul_rn(q.z, inv_t),
-      s[4 * j + 3] = __fmul_rn(q.w, inv_t);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s[4 * j + i] = (g < group_end && base + i < vocab) ? __fmul_rn(row[base + i], inv_t) : CUDART_NAN_F;
-    }
-  }
   for (int b = tid; b < FILTER_BINS; b += FILTER_THREADS) {
     row_mass[b] = 0ull;
     row_count[b] = 0u;
@@ -567,53 +572,45 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
     own_lo[b] = 0u;
     own_hi[b] = 0u;
   }
+  if (tid == 0) {
+    listed = 0u;
+    choice.digit = FILTER_BINS - 1, choice.count = 0u, choice.mass = 0ull;
+  }
   float m = -CUDART_INF_F;
-#pragma unroll
-  for (int j = 0; j < FC_PER_THREAD; ++j) m = fmaxf(m, s[j]);  // fmaxf passes over NaN
+  sweep_row(own_row, entries, vectors, [&](float x) { m = fmaxf(m, __fmul_rn(x, inv_t)); });  // fmaxf passes over NaN
   m = warp_max(m);
   if ((tid & 31) == 0) scratch[tid >> 5] = m;
   __syncthreads();
   if (tid < 32) {
-    float w = scratch[tid];
-    w = warp_max(w);
-    if (tid < FC_CLUSTER) *cluster_peer(&peer_max[rank], (unsigned int)tid) = w;
+    const float w = warp_max(scratch[tid]);
+    if (tid < CLUSTER) *cluster_peer(&peer_max[rank], (unsigned int)tid) = w;
   }
   // Every CTA's maximum is in every CTA, and CTA 0's row histogram is zero, before anyone adds.
   cluster_sync_all();
   m = peer_max[0];
 #pragma unroll
-  for (int c = 1; c < FC_CLUSTER; ++c) m = fmaxf(m, peer_max[c]);
+  for (int c = 1; c < CLUSTER; ++c) m = fmaxf(m, peer_max[c]);
   const float top = m;
 
   unsigned int* count0 = cluster_peer(row_count, 0u);
   unsigned long long* mass0 = cluster_peer(row_mass, 0u);
-  uint32_t prefix = 0u;
+  const int copy = ((tid >> 5) % FC_COPIES) * FILTER_BINS;
+  const auto count_entry = [&](int bin, float s) {
+    atomicAdd(&own_count[copy + bin], 1u);
+    if (use_p) add_mass_words(own_lo + copy, own_hi + copy, (uint32_t)bin, fixed_mass(expf(s - top)));
+  };
+  // The bins of all CTAs into the row's histogram, the digit that CTA 0 chooses into every CTA.  A CTA's own
+  // bins go back to zero; with `keep` the row's histogram stays for what is added to it next.
   DigitSearch search = {0u, 0ull, 0ull};
-  const int shifts[3] = {21, 10, 0};
-  const int bits[3] = {11, 11, 10};
-#pragma unroll
-  for (int level = 0; level < 3; ++level) {
-    const int shift = shifts[level], level_bits = bits[level];
-    const uint32_t digit_mask = (1u << level_bits) - 1u;
-    const int copies = level == 0 ? FC_COPIES : 1;
-    const int copy = level == 0 ? ((tid >> 6) % FC_COPIES) * FILTER_BINS : 0;
-#pragma unroll
-    for (int j = 0; j < FC_PER_THREAD; ++j) {
-      const float x = s[j];
-      if (!(x == x)) continue;
-      const uint32_t key = float_key(x);
-      if (level > 0 && (key >> (shift + level_bits)) != prefix) continue;
-      const uint32_t digit = (key >> shift) & digit_mask;
-      if (use_k) atomicAdd(&own_count[copy + digit], 1u);
-      if (use_p) add_mass_words(own_lo + copy, own_hi + copy, digit, fixed_mass(expf(x - top)));
-    }
+  const auto choose_in_cluster = [&](bool keep) {
     __syncthreads();
-    // This CTA's bins into the row's histogram; its own go back to zero for the next digit.
     for (int b = tid; b < FILTER_BINS; b += FILTER_THREADS) {
       unsigned int c = 0u;
       unsigned long long w = 0ull;
-      for (int i = 0; i < copies; ++i) {
+#pragma unroll
+      for (int i = 0; i < FC_COPIES; ++i) {
         const int at = i * FILTER_BINS + b;
+        if (own_count[at] == 0u) continue;
         c += own_count[at];
         w += ((unsigned long long)own_hi[at] << 32) + own_lo[at];
         own_count[at] = 0u, own_lo[at] = 0u, own_hi[at] = 0u;
@@ -625,15 +622,138 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
     if (rank == 0u) {
       const unsigned int c0 = row_count[2 * tid], c1 = row_count[2 * tid + 1];
       const unsigned long long m0 = row_mass[2 * tid], m1 = row_mass[2 * tid + 1];
-      row_count[2 * tid] = 0u, row_count[2 * tid + 1] = 0u;
-      row_mass[2 * tid] = 0ull, row_mass[2 * tid + 1] = 0ull;
-      const unsigned int digit = choose_digit(c0, c1, m0, m1, level == 0, use_k, k, use_p, p, search, sc, sm, &choice);
-      if (tid < FC_CLUSTER) *cluster_peer(&chosen_digit, (unsigned int)tid) = digit;
+      const DigitSearch before = search;
+      const unsigned int digit = choose_digit(c0, c1, m0, m1, false, use_k, k, use_p, p, search, sc, sm, &choice);
+      if (tid == (int)(digit >> 1))
+        for (unsigned int c = 0; c < CLUSTER; ++c) {
+          *cluster_peer(&chosen_digit, c) = digit;
+          *cluster_peer(&chosen_entries, c) = (digit & 1u) ? c1 : c0;
+        }
+      if (keep && digit == 0u)
+        search = before;
+      else
+        row_count[2 * tid] = row_count[2 * tid + 1] = 0u, row_mass[2 * tid] = row_mass[2 * tid + 1] = 0ull;
     }
     cluster_sync_all();
-    prefix = (prefix << level_bits) | chosen_digit;
+    return chosen_digit;
+  };
+
+  // The near entries' histogram and the mass of all.
+  constexpr int NEAR_FROM = FILTER_BINS - FC_NEAR;
+  unsigned long long total = 0ull;
+  sweep_row(own_row, entries, vectors, [&](float x) {
+    const float s = __fmul_rn(x, inv_t);
+    if (!(s == s)) return;  // NaN is never a candidate
+    const int bin = distance_bin(s, top);
+    if (use_p) {
+      const unsigned long long w = fixed_mass(expf(s - top));
+      total += w;
+      if (bin >= NEAR_FROM) add_mass_words(own_lo + copy, own_hi + copy, (uint32_t)bin, w);
+    }
+    if (bin >= NEAR_FROM) atomicAdd(&own_count[copy + bin], 1u);
+  });
+  if (use_p) {
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
+    if ((tid & 31) == 0) sm[tid >> 5] = total;
+    __syncthreads();
+    if (tid < 32) {
+      total = sm[tid];
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
+      if (tid == 0) *cluster_peer(&peer_total[rank], 0u) = total;
+    }
+    cluster_sync_all();
+    if (rank == 0u) {
+      total = 0ull;
+#pragma unroll
+      for (int c = 0; c < CLUSTER; ++c) total += peer_total[c];
+      // (At least one: the largest entry, with nothing above it, is always a candidate.)
+      search.mass_limit = max(1ull, (unsigned long long)((double)p * (double)total));
+    }
   }
-  if (rank == 0u && tid == 0) threshold[r] = key_float(prefix);
+  unsigned int bin = choose_in_cluster(true);
+  if (bin == 0u) {  // (Everything near the maximum passes.)
+    sweep_row(own_row, entries, vectors, [&](float x) {
+      const float s = __fmul_rn(x, inv_t);
+      if (!(s == s)) return;
+      const int far = distance_bin(s, top);
+      if (far < NEAR_FROM) count_entry(far, s);
+    });
+    bin = choose_in_cluster(false);
+  }
+
+  const bool no_mass = use_p && total == 0ull;  // in CTA 0: a row whose maximum is not finite
+  const unsigned int in_bin = chosen_entries;
+  if (in_bin <= (unsigned int)FC_LIST) {
+    unsigned int* list0 = cluster_peer(list_key, 0u);
+    unsigned int* listed0 = cluster_peer(&listed, 0u);
+    sweep_row(own_row, entries, vectors, [&](float x) {
+      const float s = __fmul_rn(x, inv_t);
+      if (!(s == s) || distance_bin(s, top) != (int)bin) return;
+      const unsigned int at = atomicAdd(listed0, 1u);
+      if (at < (unsigned int)FC_LIST) list0[at] = float_key(s);
+    });
+    cluster_sync_all();
+    if (rank != 0u) return;
+    const bool mine = tid < (int)in_bin;
+    const uint32_t key = mine ? list_key[tid] : 0u;
+    if (mine) list_mass[tid] = use_p ? fixed_mass(expf(key_float(key) - top)) : 0ull;
+    __syncthreads();
+    unsigned int above = search.above_count;
+    unsigned long long mass = search.above_mass;
+    if (mine)
+      for (int j = 0; j < (int)in_bin; ++j)
+        if (list_key[j] > key) above += 1u, mass += list_mass[j];
+    const bool passes = mine && (!use_k || above < (unsigned int)k) && (!use_p || mass < search.mass_limit);
+    const unsigned int smallest = __reduce_min_sync(0xffffffffu, passes ? key : 0xffffffffu);
+    if ((tid & 31) == 0) sc[tid >> 5] = smallest;
+    // Bin 0 and every entry passes: no value is too small (a row with NaN that has fewer than k entries).
+    unsigned long long bin_mass = mine && use_p ? list_mass[tid] : 0ull;
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) bin_mass += __shfl_xor_sync(0xffffffffu, bin_mass, offset);
+    if ((tid & 31) == 0) sm[tid >> 5] = bin_mass;
+    __syncthreads();
+    if (tid < 32) {
+      const unsigned int found = __reduce_min_sync(0xffffffffu, sc[tid]);
+      bin_mass = sm[tid];
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) bin_mass += __shfl_xor_sync(0xffffffffu, bin_mass, offset);
+      const bool all = bin == 0u && (!use_k || search.above_count + in_bin < (unsigned int)k) &&
+                       (!use_p || search.above_mass + bin_mass < search.mass_limit);
+      if (tid == 0) threshold[r] = no_mass ? top : all ? key_float(0u) : key_float(found);
+    }
+    return;
+  }
+
+  // Too many for a list: digit by digit over the entries of the bin.
+  uint32_t prefix = 0u;
+  const int shifts[3] = {21, 10, 0};
+  const int bits[3] = {11, 11, 10};
+#pragma unroll
+  for (int level = 0; level < 3; ++level) {
+    const int shift = shifts[level], level_bits = bits[level];
+    const uint32_t digit_mask = (1u << level_bits) - 1u;
+    sweep_row(own_row, entries, vectors, [&](float x) {
+      const float s = __fmul_rn(x, inv_t);
+      if (!(s == s) || distance_bin(s, top) != (int)bin) return;
+      const uint32_t key = float_key(s);
+      if (level > 0 && (key >> (shift + level_bits)) != prefix) return;
+      count_entry((int)((key >> shift) & digit_mask), s);
+    });
+    prefix = (prefix << level_bits) | choose_in_cluster(false);
+  }
+  if (rank == 0u && tid == 0) threshold[r] = no_mass ? top : key_float(prefix);
+}
+
+template <int CLUSTER>
+cudaError_t launch_filter_cluster(const float* logits, int num_rows, int vocab, long long row_stride, const float* temperature,
+                                  const int* top_k, const float* top_p, float* threshold, cudaStream_t stream) {
+  static const cudaError_t ready = cudaFuncSetAttribute(filter_threshold_cluster_kernel<CLUSTER>,
+                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FC_SMEM_BYTES);
+  if (ready != cudaSuccess) return ready;
+  return launch_pdl_cluster(filter_threshold_cluster_kernel<CLUSTER>, dim3((unsigned)num_rows * CLUSTER), dim3(FILTER_THREADS),
+                            FC_SMEM_BYTES, CLUSTER, stream, logits, vocab, row_stride, temperature, top_k, top_p, threshold);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -723,36 +843,15 @@ VX_API int vx_filter_threshold(const float* logits, int num_rows, int vocab, lon
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(filter_threshold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)FILTER_SMEM_BYTES);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(filter_threshold_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)FC_SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   if (kind == 2 && vocab > FC_MAX_VOCAB) return (int)cudaErrorInvalidValue;
   if (kind != 1 && vocab <= FC_MAX_VOCAB) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3((unsigned)num_rows * FC_CLUSTER);
-    config.blockDim = dim3(FILTER_THREADS);
-    config.dynamicSmemBytes = FC_SMEM_BYTES;
-    config.stream = stream;
-    cudaLaunchAttribute attributes[2];
-    int count = 0;
-    attributes[count].id = cudaLaunchAttributeClusterDimension;
-    attributes[count].val.clusterDim.x = FC_CLUSTER;
-    attributes[count].val.clusterDim.y = 1;
-    attributes[count].val.clusterDim.z = 1;
-    ++count;
-    const char* serialised = getenv("VELOX_B200_NO_PDL");
-    if (serialised == nullptr || serialised[0] != '1') {
-      attributes[count].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attributes[count].val.programmaticStreamSerializationAllowed = 1;
-      ++count;
-    }
-    config.attrs = attributes;
-    config.numAttrs = count;
-    return (int)cudaLaunchKernelEx(&config, filter_threshold_cluster_kernel, logits, vocab, row_stride, temperature,
-                                   top_k, top_p, threshold);
+    // A CTA fills an SM: the largest cluster with which all rows run at once.
+    const auto launch = num_rows * 8 <= 144 ? launch_filter_cluster<8>
+                        : num_rows * 4 <= 144 ? launch_filter_cluster<4> : launch_filter_cluster<2>;
+    return (int)launch(logits, num_rows, vocab, row_stride, temperature, top_k, top_p, threshold, stream);
   }
   launch_pdl(filter_threshold_kernel, dim3(num_rows), dim3(FILTER_THREADS), FILTER_SMEM_BYTES, stream, logits, vocab, row_stride,
                                                             temperature, top_k, top_p, threshold);

@@ -1449,8 +1449,8 @@ def filter_threshold(
 ) -> None:
     """threshold[r]: the smallest scaled logit that is a top-k / top-p candidate of row r.
 
-    ``kind`` picks the kernel: 0 a cluster of eight CTAs per row where the row fits their
-    registers (196,608 entries) and one CTA per row otherwise, 1 always one CTA per row, 2 the
+    ``kind`` picks the kernel: 0 a cluster of two, four or eight CTAs per row for rows of up to
+    196,608 entries and one CTA per row otherwise, 1 always one CTA per row, 2 the
     cluster kernel or an error.  Both give the same threshold bit for bit."""
     _need(logits, torch.float32, "logits")
     _need(temperature, torch.float32, "temperature")
