@@ -130,6 +130,21 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// True in one lane of the converged warp, the same one every time.  A warp that walks a loop as a whole
+// and issues from this lane keeps addresses and descriptors in uniform registers; in a branch of one lane
+// every tcgen05 instruction first moves its operands there.
+__device__ __forceinline__ bool elect_lane() {
+  uint32_t elected;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(elected));
+  return elected != 0u;
+}
+
 // Bulk copy global -> shared (16-byte aligned, size a multiple of 16) that signals `bar`.
 __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes,
                                               uint32_t bar) {

@@ -14,7 +14,7 @@
 //
 //   warp 0, one lane : TMA producer.  cp.async.bulk.tensor 2-D tiles of W [128 x 64] and
 //                      X [BN x 64] into a ring of 128-byte-swizzled shared-memory stages.
-//   warp 1, one lane : tcgen05.mma issuer (kind::f16, bf16 x bf16 -> f32 in TMEM), four
+//   warp 1           : tcgen05.mma issuer, from one lane (kind::f16, bf16 x bf16 -> f32 in TMEM), four
 //                      K=16 instructions per stage; tcgen05.commit frees the stage and, after
 //                      the last stage, signals the epilogue.  The warp owns the TMEM allocation.
 //   warps 2..5       : epilogue.  tcgen05.ld 32 lanes x 32 columns; a thread holds one output
@@ -394,11 +394,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       load_w(i);
       if (!normed) load_x(i);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
+    // The whole warp walks the loop and one lane issues (see elect_lane): four instructions of a K block take
+    // about 100 cycles less each than from a branch of one lane, which is on the chain of every small step
+    // (1.5B sizes, a step of 64 tokens 2,957 -> 2,542 us, of 8 tokens 1,368 -> 1,295; 0.5B sizes, one token
+    // 804 -> 716; together with the activations formed by all four warps below).
     constexpr uint32_t idesc = umma_instr_desc(BN);
+    const bool issues = elect_lane();
     bool ok = true;
-    for (int i = 0; i < num_kb && ok; ++i) {
+    for (int i = 0; i < num_kb; ++i) {
       const int stage = i % S::STAGES;
       const uint32_t phase = (uint32_t)(i / S::STAGES) & 1u;
       ok = mbar_wait(smem_u32(&full_bar[stage]), phase, g.status);
@@ -406,24 +411,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       const int batch = i / S::NORM_BATCH, ring_batches = normed ? g.x_slots / S::NORM_BATCH : 1;
       if (ok && normed && i % S::NORM_BATCH == 0)
         ok = mbar_wait(smem_u32(&x_bar[batch % ring_batches]), (uint32_t)(batch / ring_batches) & 1u, g.status);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t a_addr = smem_base + stage * S::STAGE_BYTES;
       const uint32_t b_addr = normed ? smem_base + S::STAGES * S::STAGE_BYTES + S::RECV_BYTES +
                                            (uint32_t)(i % g.x_slots) * S::B_BYTES
                                      : a_addr + GB_A_BYTES;
+      const uint64_t a_desc = umma_smem_desc(a_addr), b_desc = umma_smem_desc(b_addr);
+      if (issues) {
+        // (Sixteen of the inner dimension are 32 bytes, two units of a descriptor's address.)
 #pragma unroll
-      for (int k = 0; k < GB_BK / 16; ++k) {
-        umma_bf16(tmem_acc, umma_smem_desc(a_addr + k * 32), umma_smem_desc(b_addr + k * 32),
-                  idesc, (i > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < GB_BK / 16; ++k)
+          umma_bf16(tmem_acc, a_desc + k * 2, b_desc + k * 2, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&empty_bar[stage]));
+        // The last product of a batch: when it has finished, the batch's place is free again.
+        if (normed && (i % S::NORM_BATCH == S::NORM_BATCH - 1 || i == num_kb - 1))
+          umma_commit(smem_u32(&x_free[batch % ring_batches]));
       }
-      umma_commit(smem_u32(&empty_bar[stage]));
-      // The last product of a batch: when it has finished, the batch's place is free again.
-      if (normed && (i % S::NORM_BATCH == S::NORM_BATCH - 1 || i == num_kb - 1))
-        umma_commit(smem_u32(&x_free[batch % ring_batches]));
+      __syncwarp();
     }
     // Arrives when every MMA above has finished (or at once if there were none).
-    umma_commit(smem_u32(&acc_bar));
+    if (issues) umma_commit(smem_u32(&acc_bar));
+    __syncwarp();
   } else if (warp >= 2) {
     // ---------------------------------------------------------------- epilogue
     grid_dependency_wait();
@@ -553,22 +563,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // rows 0..63 gate, 64..127 up of the same 64 output features
         const int n = n0 + (row & 63);
         __nv_bfloat16* out = (__nv_bfloat16*)g.out;
-        const bool biased = g.bias != nullptr && row < 64 && n < g.N;
+        const bool biased = g.bias != nullptr && n < g.N;
         const float bias_gate = biased ? g.bias[n] : 0.f, bias_up = biased ? g.bias[g.N + n] : 0.f;
         for (int c0 = 0; c0 < BN; c0 += 32) {
           float v[32];
           if (BN >= 32) tmem_load_32(lane_base + c0, v); else tmem_load_16(lane_base + c0, v);
-          // up rows hand their values to the gate rows through shared memory
-          if (row >= 64) {
-            for (int j = 0; j < cols; ++j) swap_buf[(row - 64) * 33 + j] = v[j];
-          }
+          // Gate and up rows of a feature hand each other half of their tokens through shared memory, so that
+          // all four warps form activations: gate rows those of even tokens, up rows those of odd ones.
+          const bool is_up = row >= 64;
+          float* const swap = swap_buf + (row & 63) * 33;
+#pragma unroll
+          for (int j = 0; j < cols; j += 2) swap[j + (is_up ? 0 : 1)] = is_up ? v[j] : v[j + 1];
           asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (row < 64 && n < g.N) {
-            for (int j = 0; j < cols; ++j) {
+          if (n < g.N) {
+#pragma unroll
+            for (int i = 0; i < cols; i += 2) {
+              const int j = i + (is_up ? 1 : 0);
               const int t = t0 + c0 + j;
               if (t < g.T) {
                 const float scale = normed ? ssq_s[c0 + j] : 1.0f;
-                float gate = v[j] * scale + bias_gate, up = swap_buf[row * 33 + j] * scale + bias_up;
+                const float own = is_up ? v[i + 1] : v[i], other = swap[j];
+                float gate = (is_up ? other : own) * scale + bias_gate, up = (is_up ? own : other) * scale + bias_up;
                 if (g.glu_limit > 0.f) {
                   gate = fminf(gate, g.glu_limit);
                   up = fminf(fmaxf(up, -g.glu_limit), g.glu_limit);
@@ -1031,42 +1046,51 @@ mlp_fused_kernel(const __grid_constant__ CUtensorMap map_gate, const __grid_cons
       if (!mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1u, m.status)) break;
       load(i);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     constexpr uint32_t idesc = umma_instr_desc(MF_BN);
+    const bool issues = elect_lane();
     bool ok = true;
-    for (int i = 0; i < kb1 && ok; ++i) {
+    for (int i = 0; i < kb1; ++i) {
       const int stage = i % MF_STAGES;
       const uint32_t phase = (uint32_t)(i / MF_STAGES) & 1u;
       ok = mbar_wait(smem_u32(&full_bar[stage]), phase, m.status);
       if (ok && i % MF_NORM_BATCH == 0) ok = mbar_wait(smem_u32(&x_bar[i / MF_NORM_BATCH]), 0u, m.status);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_addr = smem_base + stage * GB_A_BYTES;
-      const uint32_t b_addr = x_addr + i * MF_X_BYTES;
+      const uint64_t a_desc = umma_smem_desc(smem_base + stage * GB_A_BYTES);
+      const uint64_t b_desc = umma_smem_desc(x_addr + i * MF_X_BYTES);
+      if (issues) {
 #pragma unroll
-      for (int k = 0; k < GB_BK / 16; ++k)
-        umma_bf16(tmem_acc, umma_smem_desc(a_addr + k * 32), umma_smem_desc(b_addr + k * 32), idesc,
-                  (i > 0 || k > 0) ? 1u : 0u);
-      umma_commit(smem_u32(&empty_bar[stage]));
+        for (int k = 0; k < GB_BK / 16; ++k)
+          umma_bf16(tmem_acc, a_desc + k * 2, b_desc + k * 2, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        umma_commit(smem_u32(&empty_bar[stage]));
+      }
+      __syncwarp();
     }
-    umma_commit(smem_u32(&acc1_bar));
+    if (issues) umma_commit(smem_u32(&acc1_bar));
+    __syncwarp();
     // The activation tile is the B operand of every product of the second part.
     if (ok) ok = mbar_wait(smem_u32(&act_bar), 0u, m.status);
-    for (int t2 = 0; t2 < tiles2 && ok; ++t2) {
+    const uint64_t act_desc = umma_smem_desc(act_addr);
+    for (int t2 = 0; t2 < tiles2; ++t2) {
       const int i = kb1 + t2;
       const int stage = i % MF_STAGES;
       const uint32_t phase = (uint32_t)(i / MF_STAGES) & 1u;
-      ok = mbar_wait(smem_u32(&full_bar[stage]), phase, m.status);
+      if (ok) ok = mbar_wait(smem_u32(&full_bar[stage]), phase, m.status);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t a_addr = smem_base + stage * GB_A_BYTES;
+      const uint64_t a_desc = umma_smem_desc(smem_base + stage * GB_A_BYTES);
+      if (issues) {
 #pragma unroll
-      for (int k = 0; k < GB_BK / 16; ++k)
-        umma_bf16(tmem_acc + (uint32_t)MF_BN * (1u + (uint32_t)t2), umma_smem_desc(a_addr + k * 32),
-                  umma_smem_desc(act_addr + k * 32), idesc, k > 0 ? 1u : 0u);
-      umma_commit(smem_u32(&empty_bar[stage]));
-      umma_commit(smem_u32(&tile_bar[t2]));
+        for (int k = 0; k < GB_BK / 16; ++k)
+          umma_bf16(tmem_acc + (uint32_t)MF_BN * (1u + (uint32_t)t2), a_desc + k * 2, act_desc + k * 2, idesc, k > 0 ? 1u : 0u);
+        umma_commit(smem_u32(&empty_bar[stage]));
+        umma_commit(smem_u32(&tile_bar[t2]));
+      }
+      __syncwarp();
     }
   } else if (warp >= 2) {
     // ---------------------------------------------------------------- norm, activation, output
@@ -1143,23 +1167,25 @@ mlp_fused_kernel(const __grid_constant__ CUtensorMap map_gate, const __grid_cons
 #pragma unroll
       for (int j = 0; j < MF_BN; ++j) v[j] = 0.f;
     }
-    // Rows 0..63 are gate, 64..127 up of the same 64 features: up rows hand their values over.
-    if (row >= 64) {
+    // Rows 0..63 are gate, 64..127 up of the same 64 features.  They hand each other half of their tokens: gate
+    // rows form the activations of even tokens, up rows those of odd ones.
+    const bool is_up = row >= 64;
+    const int feature = row & 63;
+    float* const swap = swap_buf + feature * (MF_BN + 1);
 #pragma unroll
-      for (int j = 0; j < MF_BN; ++j) swap_buf[(row - 64) * (MF_BN + 1) + j] = v[j];
-    }
+    for (int j = 0; j < MF_BN; j += 2) swap[j + (is_up ? 0 : 1)] = is_up ? v[j] : v[j + 1];
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (row < 64) {
-      // Activation tile [MF_BN tokens x 64 features] bf16, K-major, 128-byte swizzled: feature f
-      // of token t in chunk (f / 8) ^ (t & 7) of row t.
+    // Activation tile [MF_BN tokens x 64 features] bf16, K-major, 128-byte swizzled: feature f
+    // of token t in chunk (f / 8) ^ (t & 7) of row t.
 #pragma unroll
-      for (int j = 0; j < MF_BN; ++j) {
-        const float scale = rstd_s[j];
-        const float gate = v[j] * scale, up = swap_buf[row * (MF_BN + 1) + j] * scale;
-        const float a = j < m.T ? gate / (1.0f + __expf(-gate)) * up : 0.f;
-        *reinterpret_cast<__nv_bfloat16*>(act_tile + j * 128 + ((((row >> 3) ^ (j & 7))) << 4) + (row & 7) * 2) =
-            __float2bfloat16_rn(a);
-      }
+    for (int i = 0; i < MF_BN; i += 2) {
+      const int j = i + (is_up ? 1 : 0);
+      const float scale = rstd_s[j];
+      const float own = (is_up ? v[i + 1] : v[i]) * scale, other = swap[j] * scale;
+      const float gate = is_up ? other : own, up = is_up ? own : other;
+      const float a = j < m.T ? gate / (1.0f + __expf(-gate)) * up : 0.f;
+      *reinterpret_cast<__nv_bfloat16*>(act_tile + j * 128 + ((((feature >> 3) ^ (j & 7))) << 4) + (feature & 7) * 2) =
+          __float2bfloat16_rn(a);
     }
     // The tensor core reads the tile through the async proxy.
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
