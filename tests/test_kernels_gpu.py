@@ -1005,7 +1005,19 @@ def test_gemm_bf16_swiglu_makes_its_input_norm(k, status, T, I, K):
 def test_gemm_bf16_qkv_rotates_and_writes_the_cache(k, status, T, H, G, K, normed):
     """Heads of 128 dims: the QKV projection rotates q and k by the tokens' positions and writes
     k and v into the paged cache in its epilogue (and makes its input norm, if asked)."""
-    D, P = 128, 16
+    check_qkv_rope(k, status, T, H, G, K, normed, 128)
+
+
+@pytest.mark.parametrize("T,H,G,K,D", [(1, 14, 2, 896, 64), (33, 3, 1, 512, 64), (4, 8, 1, 256, 32), (64, 5, 2, 320, 32),
+                                       (17, 7, 3, 256, 16)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_gemm_bf16_qkv_rotates_smaller_heads(k, status, T, H, G, K, D, normed):
+    """Two, four and eight heads to a tile of 128 rows, the last tile not full."""
+    check_qkv_rope(k, status, T, H, G, K, normed, D)
+
+
+def check_qkv_rope(k, status, T, H, G, K, normed, D):
+    P = 16
     gen = torch.Generator().manual_seed(T + H + K)
     N = (H + 2 * G) * D
     w = (torch.randn(N, K, generator=gen) / math.sqrt(K)).to(torch.bfloat16).cuda()
@@ -1039,7 +1051,7 @@ def test_gemm_bf16_qkv_rotates_and_writes_the_cache(k, status, T, H, G, K, norme
     assert int(status[0]) == 0
     y = (x64 @ w.double().T + bias.double()).cpu().view(T, H + 2 * G, D)
     c64, s64 = angles.cos().double()[positions.long()], angles.sin().double()[positions.long()]  # [T, 64]
-    lo, hi = y[..., :64], y[..., 64:]
+    lo, hi = y[..., : D // 2], y[..., D // 2:]
     rot = torch.cat([lo * c64[:, None] - hi * s64[:, None], lo * s64[:, None] + hi * c64[:, None]], dim=-1)
     want_q, want_k, want_v = rot[:, :H], rot[:, H:H + G], y[:, H + G:]
     scale = max(y.abs().max().item(), 1.0)

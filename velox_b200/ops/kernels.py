@@ -112,7 +112,7 @@ def core():
         ]
         lib.vx_gemm_bf16_qkv_rope.argtypes = [
             _ptr, _c_int, _ptr, _c_ll, _ptr, _c_f, _ptr, _ptr, _ptr, _c_int, _c_int, _c_ll, _c_int,
-            _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _c_ll, _c_int, _c_int, _ptr, _ptr,
+            _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _c_ll, _c_int, _c_int, _c_int, _ptr, _ptr,
         ]
         _core = lib
     return _core
@@ -1138,6 +1138,13 @@ def mlp_fused(
     return True
 
 
+def qkv_rope_head_dim(width: int, num_heads: int, num_kv_heads: int) -> Optional[int]:
+    """Dims of a head of a q | k | v projection of this width, if ``gemm_bf16_qkv_rope`` takes them: whole
+    heads fill a tile of 128 rows."""
+    dims, rest = divmod(width, num_heads + 2 * num_kv_heads)
+    return dims if rest == 0 and dims in (16, 32, 64, 128) else None
+
+
 def gemm_bf16_qkv_rope(
     x: Optional[torch.Tensor],
     resid: Optional[torch.Tensor],
@@ -1158,8 +1165,8 @@ def gemm_bf16_qkv_rope(
     status: torch.Tensor,
     splits: int,
 ) -> bool:
-    """The QKV projection of heads of 128 dims with rotate-half RoPE and the cache write in its
-    epilogue: rotated queries go to ``out`` [rows, (heads + 2 kv_heads) * 128] (its key and
+    """The QKV projection of heads of 16, 32, 64 or 128 dims with rotate-half RoPE and the cache write in
+    its epilogue: rotated queries go to ``out`` [rows, (heads + 2 kv_heads) * dims] (its key and
     value columns are left as they are), rotated keys and the values into the paged caches at
     ``slots`` (None caches: no write).  The input is ``x`` (bfloat16) or, when ``resid`` is
     given, ``rmsnorm(resid) * norm_weight``.  False, with nothing launched, for shapes the
@@ -1171,7 +1178,8 @@ def gemm_bf16_qkv_rope(
     _need(cos, torch.float32, "cos")
     _need(sin, torch.float32, "sin")
     n, k = w.shape
-    if n != (num_heads + 2 * num_kv_heads) * 128 or out.shape[1] != n or cos.shape[1] != 64:
+    head_dim = qkv_rope_head_dim(n, num_heads, num_kv_heads)
+    if head_dim is None or out.shape[1] != n or cos.shape[1] * 2 != head_dim:
         return False
     if num_rows > GEMM_NORMED_MAX_TOKENS:
         return False
@@ -1187,14 +1195,14 @@ def gemm_bf16_qkv_rope(
     if write:
         _need(k_cache, torch.bfloat16, "k_cache")
         _need(v_cache, torch.bfloat16, "v_cache")
-        if k_cache.shape[2] != num_kv_heads or k_cache.shape[3] != 128:
+        if k_cache.shape[2] != num_kv_heads or k_cache.shape[3] != head_dim:
             return False
     num_slots = k_cache.shape[0] * k_cache.shape[1] if write else 0
     code = core().vx_gemm_bf16_qkv_rope(
         _p(x), 0 if x is None else x.shape[0], _p(resid), 0 if resid is None else resid.stride(0),
         _p(norm_weight), float(eps), _p(w), _p(bias), _p(out), num_rows, k, out.stride(0), splits,
         _p(positions), _p(cos), _p(sin), cos.shape[0], _p(slots), _p(k_cache), _p(v_cache), num_slots,
-        num_heads, num_kv_heads, _p(status), _stream())
+        num_heads, num_kv_heads, head_dim, _p(status), _stream())
     if code in (-1, -2):
         return False
     _check(code, "gemm_bf16_qkv_rope")

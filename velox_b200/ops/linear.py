@@ -220,12 +220,14 @@ def qkv_rope_linear(
     num_kv_heads: int,
 ) -> bool:
     """The QKV projection with the rotation of q and k and the write of k and v into the cache
-    in the same kernel (few tokens, heads of 128 dims, a projection that is split along K).
+    in the same kernel (few tokens, heads that fill tiles of 128 rows, a projection that is split along K).
     ``x`` is a tensor or a ``PendingNorm``.  False: nothing was done; the caller projects with
     ``linear`` and rotates with the position part."""
     if status is None or num_rows == 0 or num_rows > kernels.GEMM_NORMED_MAX_TOKENS:
         return False
-    if not use_tensor_core_kernel(x, weight, num_rows):
+    # (Asked before anything runs: the caller's own projection can make a pending norm as well.)
+    if not use_tensor_core_kernel(x, weight, num_rows) or kernels.qkv_rope_head_dim(
+            weight.shape[0], num_heads, num_kv_heads) is None:
         return False
     splits = choose_splits(weight.shape[0], weight.shape[1], num_rows)
     if splits < 2:
