@@ -197,11 +197,21 @@ def test_gemm_f32_every_tile_sums_alike(k, N, K, offset):
         assert torch.all(out[M] == 5.0)
 
 
+@pytest.mark.parametrize("hidden,T", [(5120, 300), (5124, 256), (8192, 257), (8196, 256)])
+def test_add_rmsnorm_many_wide_rows(k, hidden, T):
+    """Eight warps a row up to 8,192 elements, and the rows beyond."""
+    check_add_rmsnorm(k, torch.bfloat16, hidden, T)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,T", [(1536, 700), (3584, 300), (240, 513), (4100, 260)])
 def test_add_rmsnorm_many_rows(k, dtype, hidden, T):
     """Steps of many rows (a warp per row in bfloat16), with and without rows to add, selected
     rows, and a tail that does not fill the last block."""
+    check_add_rmsnorm(k, dtype, hidden, T)
+
+
+def check_add_rmsnorm(k, dtype, hidden, T):
     gen = torch.Generator().manual_seed(hidden + T)
     resid = (torch.randn(T + 2, hidden, generator=gen) * 3).cuda()
     delta = torch.randn(T + 2, hidden, generator=gen).to(dtype).cuda()

@@ -641,14 +641,18 @@ VX_API int vx_add_rmsnorm(float* resid, const void* delta, const float* weight, 
   if (num_out_rows <= 0) return 0;
   const bool aligned = (reinterpret_cast<uintptr_t>(resid) & 15) == 0 && (reinterpret_cast<uintptr_t>(weight) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (reinterpret_cast<uintptr_t>(delta) & 15) == 0;
-  // Many rows: a few warps per row (rows of up to 4,096 elements, whole chunks of four).  Not in
+  // Many rows: a few warps per row (rows of up to 8,192 elements, whole chunks of four).  Not in
   // the float32 path: there a row's sum of squares is added up in the same order whatever the
   // step, so that results do not depend on how the work was cut.
-  if (aligned && dtype == VX_DTYPE_BF16 && num_out_rows >= 256 && hidden % 4 == 0 && hidden <= 4096) {
+  if (aligned && dtype == VX_DTYPE_BF16 && num_out_rows >= 256 && hidden % 4 == 0 && hidden <= 8192) {
     // Four warps a row (measured in a prefill of the 1.5B sizes: 9.1 us a launch at 2,048 rows
     // with one warp a row, 7.9 with two, 6.8 with four, 7.3 with eight; 8.5 -> 3.1 us at 512 rows).
     if (hidden <= 2048) launch_rmsnorm_warp<__nv_bfloat16, 4, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
-    else launch_rmsnorm_warp<__nv_bfloat16, 8, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
+    else if (hidden <= 4096) launch_rmsnorm_warp<__nv_bfloat16, 8, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
+    // Eight warps a row beyond that, five chunks a lane at 5,120 elements (a block of 1,024 threads a row before:
+    // 28.6 us a launch at 2,048 rows; the 14B sizes' portion of 2,048 tokens 71.9 -> 71.3 ms).
+    else if (hidden <= 5120) launch_rmsnorm_warp<__nv_bfloat16, 5, 8>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
+    else launch_rmsnorm_warp<__nv_bfloat16, 8, 8>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
     return (int)cudaGetLastError();
   }
   if (aligned && hidden % 4 == 0 && hidden / 4 <= 1024 * NORM_VEC_CHUNKS) {
