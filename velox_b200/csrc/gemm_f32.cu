@@ -82,8 +82,12 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
   constexpr int TM = S::thread_m, TN = S::thread_n, STAGES = S::STAGES;
   constexpr int STEP_M = S::lanes_m * S::warps_m, STEP_N = S::LN * S::warps_n;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row_m = (warp % S::warps_m) * S::lanes_m + lane / S::LN;
-  const int row_n = (warp / S::warps_m) * S::LN + lane % S::LN;
+  // Neighbouring lanes read the same weights, and a quarter of a warp two rows of A: a 16-byte read of a
+  // warp then takes two passes over the banks where lanes 0 ... 7 with eight rows took four.
+  const int lane_m = S::lanes_m == 4 ? (lane & 1) | ((lane >> 4) << 1) : lane / S::LN;
+  const int lane_n = S::lanes_m == 4 ? (lane >> 1) & 7 : lane % S::LN;
+  const int row_m = (warp % S::warps_m) * S::lanes_m + lane_m;
+  const int row_n = (warp / S::warps_m) * S::LN + lane_n;
   // x: the ranges of K, so that a cluster is one output tile; y: tiles of N; z: tiles of M.
   const int rank = blockIdx.x;
   const int n0 = blockIdx.y * S::BN, m0 = blockIdx.z * S::BM;
