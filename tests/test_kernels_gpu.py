@@ -742,6 +742,33 @@ def test_filter_threshold_clusters_of_every_size(k, rows):
     assert torch.equal(one.view(torch.int32), auto.view(torch.int32)), (one.tolist(), auto.tolist())
 
 
+@pytest.mark.parametrize("vocab,kinds", [(9, (1, 2)), (50021, (1, 2)), (196608 + 40, (0, 1))])
+def test_filter_threshold_of_rows_without_mass(k, vocab, kinds):
+    """A top_p below the masses' resolution and rows whose maximum is not finite: the largest entry is a
+    candidate in every form, whatever ran on the SM before."""
+    inf, nan = float("inf"), float("nan")
+    logits = torch.randn(8, vocab, generator=torch.Generator().manual_seed(vocab))
+    logits[1, [2, 5]] = inf  # (two entries' masses, 2^63 each, add up to zero)
+    logits[2, 4] = inf
+    logits[3, [0, 4, 7]] = inf
+    logits[4] = -inf
+    logits[5] = nan
+    logits[6, 1:] = nan
+    logits[7, [2, 5]] = inf
+    top_p = torch.tensor([1e-13, 0.9, 0.9, 0.3, 0.9, 0.9, 0.9, 0.5])
+    top_k = torch.tensor([0, 0, 0, 0, 0, 0, 0, 3], dtype=torch.int32)
+    want = torch.tensor([logits[0].max().item(), inf, inf, inf, -inf, -inf, logits[6, 0].item(), inf])
+    for kind in kinds:
+        for _ in range(3):
+            # Leaves bins of another row in the shared memory that the next launch finds.
+            other = torch.randn(300, 5000, device="cuda")
+            k.filter_threshold(other, 300, torch.ones(300).cuda(), torch.full((300,), 9, dtype=torch.int32).cuda(),
+                               torch.full((300,), 0.9).cuda(), torch.empty(300, device="cuda"), kind=1)
+            thr = torch.full((8,), 7.0, device="cuda")
+            k.filter_threshold(logits.cuda(), 8, torch.ones(8).cuda(), top_k.cuda(), top_p.cuda(), thr, kind=kind)
+            assert torch.equal(thr.cpu(), want), (kind, thr.tolist(), want.tolist())
+
+
 def test_filter_threshold_beyond_the_cluster_kernel(k):
     """A row longer than the cluster's registers hold takes the one-CTA kernel; asking for the
     cluster kernel by name is refused."""

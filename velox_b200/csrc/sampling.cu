@@ -312,7 +312,8 @@ __device__ __forceinline__ unsigned int choose_digit(unsigned int c0, unsigned i
   if (first) {
     if (threadIdx.x == 0) choice->total = m_above + m0 + m1;
     __syncthreads();
-    search.mass_limit = (unsigned long long)((double)p * (double)choice->total);
+    // (At least one: the largest entry, with nothing above it, is always a candidate.)
+    search.mass_limit = max(1ull, (unsigned long long)((double)p * (double)choice->total));
   }
   const unsigned int c_hi = search.above_count + c_above, c_lo = c_hi + c1;  // above digit 2t + 1, above 2t
   const unsigned long long m_hi = search.above_mass + m_above, m_lo = m_hi + m1;
@@ -457,6 +458,10 @@ filter_threshold_kernel(const float* __restrict__ logits, int vocab, long long r
         w[i] += hist_mass[copy * FILTER_BINS + 2 * threadIdx.x + i];
       }
     const unsigned int digit = choose_digit(c[0], c[1], w[0], w[1], level == 0, use_k, k, use_p, p, search, sc, sm, &choice);
+    if (use_p && choice.total == 0ull) {  // no mass at all: a row whose maximum is not finite
+      if (threadIdx.x == 0) threshold[r] = m;
+      return;
+    }
     prefix = (prefix << bits[level]) | digit;
     __syncthreads();
   }
