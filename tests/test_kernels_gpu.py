@@ -742,6 +742,38 @@ def test_filter_threshold_clusters_of_every_size(k, rows):
     assert torch.equal(one.view(torch.int32), auto.view(torch.int32)), (one.tolist(), auto.tolist())
 
 
+@pytest.mark.parametrize("vocab", [300, 9001, 151936])
+@pytest.mark.parametrize("rows", [12, 24, 48])  # eight, four and two CTAs a row
+def test_filter_threshold_bounds_of_the_histogram(k, rows, vocab):
+    """k at the counts of warps and threads that the first histogram's reach follows from, top_p whose threshold
+    is near, further down and at the end of the row, lists and bins that have to be narrowed first (a thousand
+    entries within a hair, ties by the thousand), outliers and masked rows: as one CTA a row finds it."""
+    gen = torch.Generator().manual_seed(vocab + rows)
+    logits = torch.randn(rows, vocab, generator=gen) * 2
+    wide = [r for r in range(rows) if r % 12 == 1]
+    logits[wide] *= 15
+    logits[2::12, 7] = 400.0
+    logits[3::12] = 2 + 1e-4 * torch.rand(logits[3::12].shape, generator=gen)  # a few patterns apart
+    logits[3::12, ::2] -= 6
+    logits[4::12] = logits[4::12].to(torch.bfloat16).float()
+    logits[5::12, vocab // 10:] = float("-inf")
+    logits[6::12, vocab // 10:] = torch.finfo(torch.float32).min
+    logits[7::12] = (logits[7::12] * 2).round()
+    logits[8::12, 3:] = float("nan")
+    logits[9::12] = 0.3 * logits[9::12]
+    logits = logits.cuda()
+    temps = torch.tensor([0.1, 0.7, 1.3])[torch.arange(rows) // 12 % 3].cuda()
+    for top_k, top_p in ((1, 1.0), (64, 1.0), (65, 1.0), (128, 1.0), (129, 0.9), (256, 1.0), (257, 1.0), (2048, 1.0), (2049, 1.0),
+                         (4097, 0.99), (8192, 1.0), (8193, 1.0), (0, 0.5), (0, 0.9), (0, 0.99), (0, 0.99999), (50, 0.9),
+                         (vocab - 1, 1.0), (vocab - 1, 0.9999999)):
+        ks = torch.full((rows,), top_k, dtype=torch.int32).cuda()
+        ps = torch.full((rows,), top_p).cuda()
+        one, auto = (torch.full((rows,), 7.0, device="cuda") for _ in range(2))
+        k.filter_threshold(logits, rows, temps, ks, ps, one, kind=1)
+        k.filter_threshold(logits, rows, temps, ks, ps, auto)
+        assert torch.equal(one.view(torch.int32), auto.view(torch.int32)), (top_k, top_p, one.tolist(), auto.tolist())
+
+
 @pytest.mark.parametrize("vocab,kinds", [(9, (1, 2)), (50021, (1, 2)), (196608 + 40, (0, 1))])
 def test_filter_threshold_of_rows_without_mass(k, vocab, kinds):
     """A top_p below the masses' resolution and rows whose maximum is not finite: the largest entry is a
@@ -770,7 +802,7 @@ def test_filter_threshold_of_rows_without_mass(k, vocab, kinds):
 
 
 def test_filter_threshold_beyond_the_cluster_kernel(k):
-    """A row longer than the cluster's registers hold takes the one-CTA kernel; asking for the
+    """A row longer than a cluster takes goes to the one-CTA kernel; asking for the
     cluster kernel by name is refused."""
     vocab, R = 196608 + 40, 2
     gen = torch.Generator().manual_seed(3)

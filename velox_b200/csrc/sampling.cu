@@ -471,27 +471,53 @@ filter_threshold_kernel(const float* __restrict__ logits, int vocab, long long r
 // ---------------------------------------------------------------------------------------------
 // The same threshold by a cluster of CTAs per row, for rows of up to 196,608 entries.  What bounds it is
 // not the row's bytes (the head has just written them, they are in the L2) but the atomics of entries that
-// share a bin, and the waves of CTAs: so the first histogram is over the distance from the row's maximum,
-// in steps of 1/64, which spreads the entries over hundreds of bins (sign, exponent and two bits of the
-// mantissa put them into a few dozen), and at first it takes only the entries within eight units of the
-// maximum.  The mass of all the others is part of the normaliser, a sum in registers; only when the
-// threshold is not among the near entries are the far ones put into the histogram as well.  The entries of
-// the bin that holds the threshold, a few hundred as a rule, are gathered in the cluster's first CTA, which
-// looks at each: the smallest of them with fewer than k entries and less than top_p of the mass above it.
-// (A threshold is always the value of an entry, since nothing changes between two of them.)  A bin of more
-// than FC_LIST entries is searched digit by digit as in the kernel above.
+// share a bin, the cluster's meetings, and the waves of CTAs.
+//
+// One histogram finds the threshold's bin, and it takes only entries that can matter.  Each of n groups of
+// threads has an entry that is no smaller than the smallest of the groups' maxima, so at least n entries lie at
+// or above that bound: for groups of 32, 8 or 1 threads, the k-th largest entry is not below the bound of the
+// largest groups of which there are k.  And vocab entries that lie w below the maximum have at most
+// vocab * exp(-w) of its mass together: where that is less than the 1 - p of the normaliser that top_p leaves
+// out, the threshold is not below.  The normaliser is at least the maximum's own mass; where that says little (no
+// k, and a maximum that does not stand out) a pass that only sums up the mass comes first.  The bins are steps of
+// equal width between the larger of the bounds and the maximum.  With top_p and a bound that is far down the
+// histogram begins with the entries nearer by, and takes the others only if the threshold is not among those.
+// The entries of the threshold's bin, a few hundred at most as a rule, are gathered in the cluster's first CTA,
+// which looks for the smallest of them with fewer than k entries and less than top_p of the mass above it.  (A
+// threshold is always the value of an entry, since nothing changes between two of them.)  A bin of more than
+// FC_LIST entries is narrowed by the range of its patterns first.
 //
 // All sums are of the same integers as above and the histogram's bins are in the order of the values, so
 // every form gives the same threshold bit for bit.
+//
+// Measured (us a launch, 151,936 normal logits of deviation 2, in the L2; in brackets a fixed window of eight
+// units in 1/64 with rows read again for every pass and 18 rows in clusters of eight, and before that three
+// digits of the pattern over a row in registers, always eight CTAs):
+//                                  1 row              18 rows            64 rows
+//   T 0.1, top_k 200               11.4 (36.4, 17.7)  17.1 (52.6, 34.9)  22.7 (72.2, 86.6)
+//   T 0.7, top_k 200               11.4 (12.4, 17.8)  17.1 (25.1, 34.7)  22.7 (28.9, 86.6)
+//   T 0.7, top_k 50, top_p 0.9     15.6 (15.7, 20.3)  20.2 (33.3, 40.7)  27.9 (43.0, 101)
+//   T 0.7, top_p 0.99              21.7 (29.6, 23.1)  33.7 (57.1, 46.5)  52.5 (71.0, 115)
+//   T 1.2, top_p 0.9               22.4 (27.2, 23.3)  34.7 (47.9, 46.1)  53.6 (79.7, 115)
 //
 // A 64-bit sum in shared memory is a compare-and-swap loop; the masses (41 bits at most) are
 // therefore added as two 32-bit words, the low word's carry found from the value it held before.
 // ---------------------------------------------------------------------------------------------
 constexpr int FC_MAX_VOCAB = 196608;
+constexpr int FC_SHARE = FC_MAX_VOCAB / 8;  // most entries of a CTA that keeps its share
 constexpr int FC_COPIES = 2;
-constexpr int FC_LIST = 1024;          // entries of the threshold's bin that are looked at one by one
-constexpr float FC_STEPS = 64.0f;      // bins per unit of distance from the maximum
-constexpr int FC_NEAR = 8 * 64;        // bins that the first histogram fills
+constexpr int FC_LIST = 1024;          // most entries of a bin that are gathered (an entry a thread)
+constexpr int FC_PAIRS = 128;          // most entries that are compared with one another
+// Bins of the first histogram.  Every one that is not empty is added to CTA 0's by every CTA (1,024: T 0.7 with
+// top_k 1,000 and top_p 19.0 us for 18.4); in fewer, more entries share one (256: T 1.2, top_p 0.9 28.1 for 22.1).
+constexpr int FC_STEPS = 512;
+// A maximum stands out if one of 256 parts of the row (512 with four CTAs) has no entry within this distance:
+// about a hundredth of the row is nearer then.
+constexpr float FC_STANDS_OUT = 9.0f;
+// Where the histogram begins with both filters, and with top_p alone which part of the way to the bound.  (A
+// threshold further down costs a second round, 5 - 8 us; 0.6 for 0.75 had it at T 0.7, deviation 4, top_p 0.99.)
+constexpr float FC_NEAR = 8.0f;
+constexpr float FC_PART = 0.75f;
 constexpr size_t FC_SMEM_BYTES = (size_t)FILTER_BINS * (sizeof(unsigned long long) + sizeof(unsigned int)) +
                                  (size_t)FC_LIST * (sizeof(unsigned long long) + sizeof(unsigned int)) +
                                  (size_t)FC_COPIES * FILTER_BINS * 3 * sizeof(unsigned int);
@@ -506,11 +532,6 @@ __device__ __forceinline__ void add_mass_words(unsigned int* lo, unsigned int* h
   if (wh != 0u) atomicAdd(&hi[bin], wh);
 }
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // The address, in this CTA's window onto the cluster's shared memory, of `local` in CTA `rank`.
 template <typename T>
 __device__ __forceinline__ T* cluster_peer(T* local, unsigned int rank) {
@@ -519,23 +540,27 @@ __device__ __forceinline__ T* cluster_peer(T* local, unsigned int rank) {
   return reinterpret_cast<T*>(out);
 }
 
-// The bin of a value: bin FILTER_BINS - 1 starts at the row's maximum.  Monotone in s, infinities included.
-__device__ __forceinline__ int distance_bin(float s, float top) {
-  const float steps = s == top ? 0.f : fminf((top - s) * FC_STEPS, (float)(FILTER_BINS - 1));
-  return FILTER_BINS - 1 - (int)steps;
+// How far below the maximum an entry can be and still be the threshold of top_p, for a normaliser of `total`
+// times the maximum's own mass.  (The margin covers the rounding here; the masses are rounded down.)
+__device__ __forceinline__ float mass_reach(int vocab, float p, float total) {
+  return logf(fmaxf((float)vocab / ((1.0f - p) * total), 1.0f)) + 0.02f;
 }
 
-template <int CLUSTER>
+// Patterns lo ... hi cut into at most FILTER_BINS ranges of 2^shift.
+__device__ __forceinline__ int pattern_shift(uint32_t lo, uint32_t hi) { return max(0, 21 - __clz(hi - lo)); }
+
+// HELD: a CTA keeps its share of the row in shared memory; else every pass reads it again.
+template <int CLUSTER, bool HELD>
 __global__ void __launch_bounds__(FILTER_THREADS, 1)
 filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, long long row_stride,
                                 const float* __restrict__ temperature, const int* __restrict__ top_k,
                                 const float* __restrict__ top_p, float* __restrict__ threshold) {
-  __shared__ float scratch[32];
+  __shared__ float warp_least[5][32], peer_least[CLUSTER][5];
   __shared__ unsigned int sc[32];
   __shared__ unsigned long long sm[32];
-  __shared__ float peer_max[CLUSTER];
   __shared__ unsigned long long peer_total[CLUSTER];
-  __shared__ unsigned int chosen_digit, chosen_entries, listed;
+  __shared__ uint2 peer_range[CLUSTER];
+  __shared__ unsigned int chosen_digit, chosen_entries, chosen_all, listed;
   __shared__ DigitChoice choice;
   extern __shared__ __align__(16) unsigned char filter_smem[];
   unsigned long long* row_mass = reinterpret_cast<unsigned long long*>(filter_smem);   // [BINS], used in CTA 0
@@ -550,13 +575,13 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
   unsigned int rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int r = blockIdx.x / CLUSTER;
-  const int tid = (int)threadIdx.x;
+  const int tid = (int)threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float temp = temperature[r];
   const int k = top_k[r];
   const float p = top_p[r];
   const bool use_k = k > 0 && k < vocab;
   const bool use_p = p < 1.0f;
-  // The same for every CTA of the cluster: none is left waiting at a barrier.
+  // A property of the row: all CTAs of the cluster leave here or none does.
   if (temp == 0.f || (!use_k && !use_p)) {
     if (rank == 0u && tid == 0) threshold[r] = -CUDART_INF_F;
     return;
@@ -567,6 +592,38 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
   const int begin = min(vocab, (int)rank * share), entries = min(vocab, begin + share) - begin;
   const float* own_row = logits + (size_t)r * row_stride + begin;
   const bool vectors = (reinterpret_cast<uintptr_t>(own_row) & 15) == 0;
+
+  // Calls f(scaled entry) for this thread's entries, the same ones every time (and for NaN past the row's end,
+  // which nothing below counts).
+  float4* held = reinterpret_cast<float4*>(own_hi + FC_COPIES * FILTER_BINS);
+  const auto for_each = [&](auto&& f) {
+    if constexpr (HELD) {
+#pragma unroll 2
+      for (int i = tid; i < (entries + 3) >> 2; i += FILTER_THREADS) {
+        const float4 q = held[i];
+        f(q.x), f(q.y), f(q.z), f(q.w);
+      }
+    } else {
+      sweep_row(own_row, entries, vectors, [&](float x) { f(__fmul_rn(x, inv_t)); });
+    }
+  };
+  if constexpr (HELD) {
+#pragma unroll
+    for (int j = 0; j < FC_SHARE / 4 / FILTER_THREADS; ++j) {
+      const int i = j * FILTER_THREADS + tid;
+      if (4 * i >= entries) break;
+      float4 q;
+      if (vectors && 4 * i + 4 <= entries) {
+        q = reinterpret_cast<const float4*>(own_row)[i];
+      } else {
+        q.x = own_row[4 * i];
+        q.y = 4 * i + 1 < entries ? own_row[4 * i + 1] : CUDART_NAN_F;
+        q.z = 4 * i + 2 < entries ? own_row[4 * i + 2] : CUDART_NAN_F;
+        q.w = 4 * i + 3 < entries ? own_row[4 * i + 3] : CUDART_NAN_F;
+      }
+      held[i] = make_float4(__fmul_rn(q.x, inv_t), __fmul_rn(q.y, inv_t), __fmul_rn(q.z, inv_t), __fmul_rn(q.w, inv_t));
+    }
+  }
 
   for (int b = tid; b < FILTER_BINS; b += FILTER_THREADS) {
     row_mass[b] = 0ull;
@@ -581,32 +638,102 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
     listed = 0u;
     choice.digit = FILTER_BINS - 1, choice.count = 0u, choice.mass = 0ull;
   }
-  float m = -CUDART_INF_F;
-  sweep_row(own_row, entries, vectors, [&](float x) { m = fmaxf(m, __fmul_rn(x, inv_t)); });  // fmaxf passes over NaN
-  m = warp_max(m);
-  if ((tid & 31) == 0) scratch[tid >> 5] = m;
-  __syncthreads();
-  if (tid < 32) {
-    const float w = warp_max(scratch[tid]);
-    if (tid < CLUSTER) *cluster_peer(&peer_max[rank], (unsigned int)tid) = w;
-  }
-  // Every CTA's maximum is in every CTA, and CTA 0's row histogram is zero, before anyone adds.
-  cluster_sync_all();
-  m = peer_max[0];
+  // The largest entry, the smallest maximum of 32, 8 and 1 threads, and the smallest entry above -inf: five minima.
+  float most = -CUDART_INF_F, least = CUDART_INF_F;
+  for_each([&](float s) {  // (passing over NaN)
+    most = fmaxf(most, s);
+    if (s > -CUDART_INF_F) least = fminf(least, s);
+  });
+  float of_8 = most;
 #pragma unroll
-  for (int c = 1; c < CLUSTER; ++c) m = fmaxf(m, peer_max[c]);
-  const float top = m;
+  for (int offset = 1; offset < 8; offset <<= 1) of_8 = fmaxf(of_8, __shfl_xor_sync(0xffffffffu, of_8, offset));
+  const float of_32 = warp_max(of_8);
+  of_8 = -warp_max(-of_8), most = -warp_max(-most), least = -warp_max(-least);
+  if (lane == 0) {
+    warp_least[0][warp] = -of_32, warp_least[1][warp] = of_32;
+    warp_least[2][warp] = of_8, warp_least[3][warp] = most, warp_least[4][warp] = least;
+  }
+  __syncthreads();
+  if (warp < 5) {
+    const float mine = -warp_max(-warp_least[warp][lane]);
+    if (lane < CLUSTER) *cluster_peer(&peer_least[rank][warp], (unsigned int)lane) = mine;
+  }
+  // Everybody's minima are in every CTA, and CTA 0's row histogram is zero, before anyone adds.
+  cluster_meet();
+  const auto least_of = [&](int i) {
+    float v = peer_least[0][i];
+#pragma unroll
+    for (int c = 1; c < CLUSTER; ++c) v = fminf(v, peer_least[c][i]);
+    return v;
+  };
+  const float top = -least_of(0);
+  least = least_of(4);
+  if (use_p && !(fabsf(top) < CUDART_INF_F)) {
+    if (rank == 0u && tid == 0) threshold[r] = top;
+    return;
+  }
+
+  // No threshold lies below `lowest` (unless every entry passes).
+  const float of_warps = least_of(1), of_eighths = least_of(2);
+  float lowest = -CUDART_INF_F;
+  if (use_k && k <= CLUSTER * 32)
+    lowest = fmaxf(lowest, of_warps);
+  else if (use_k && k <= CLUSTER * 128)
+    lowest = fmaxf(lowest, of_eighths);
+  else if (use_k && k <= CLUSTER * 1024)
+    lowest = fmaxf(lowest, least_of(3));
+  const auto mass_of = [&](float s) { return use_p ? fixed_mass(expf(s - top)) : 0ull; };
+  DigitSearch search = {0u, 0ull, 0ull};
+  unsigned long long total = 0ull;
+  // The mass of the row from the threads' sums, in every CTA.
+  const auto share_total = [&] {
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
+    if (lane == 0) sm[warp] = total;
+    __syncthreads();
+    if (tid < 32) {
+      total = sm[tid];
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
+      if (tid < CLUSTER) *cluster_peer(&peer_total[rank], (unsigned int)tid) = total;
+    }
+    cluster_meet();
+    total = 0ull;
+#pragma unroll
+    for (int c = 0; c < CLUSTER; ++c) total += peer_total[c];
+    // (At least one: the largest entry, with nothing above it, is always a candidate.)
+    search.mass_limit = max(1ull, (unsigned long long)((double)p * (double)total));
+  };
+  const bool stands_out = (CLUSTER == 8 ? of_warps : of_eighths) < top - FC_STANDS_OUT;
+  const bool total_first = use_p && !(use_k && k <= CLUSTER * 1024) && !stands_out;
+  if (total_first) {
+    for_each([&](float s) {
+      if (s == s) total += mass_of(s);  // NaN is never a candidate
+    });
+    share_total();
+  }
+  const auto reach = [&] { return top - mass_reach(vocab, p, (float)total / FILTER_MASS_SCALE); };
+  if (use_p) lowest = fmaxf(lowest, total_first ? reach() : top - mass_reach(vocab, p, 1.0f));
+  // Where the histogram begins.
+  float near = fmaxf(lowest, least);
+  if (use_p && !total_first) near = fmaxf(lowest, top - (use_k ? FC_NEAR : FC_PART * mass_reach(vocab, p, 1.0f)));
+  const float window = top - fmaxf(lowest, least);
+  const float steps = window > 0.f && window < CUDART_INF_F ? fminf((float)FC_STEPS / window, 1e30f) : (float)FC_STEPS / 32.f;
+  // The bin of a value: the last one starts at the row's maximum.  Monotone in s, infinities included.
+  const auto bin_of = [&](float s) {
+    return FILTER_BINS - 1 - (s == top ? 0 : (int)fminf((top - s) * steps, (float)(FC_STEPS - 1)));
+  };
 
   unsigned int* count0 = cluster_peer(row_count, 0u);
   unsigned long long* mass0 = cluster_peer(row_mass, 0u);
-  const int copy = ((tid >> 5) % FC_COPIES) * FILTER_BINS;
-  const auto count_entry = [&](int bin, float s) {
+  const int copy = (warp % FC_COPIES) * FILTER_BINS;
+  const auto count_entry = [&](int bin, unsigned long long w) {
     atomicAdd(&own_count[copy + bin], 1u);
-    if (use_p) add_mass_words(own_lo + copy, own_hi + copy, (uint32_t)bin, fixed_mass(expf(s - top)));
+    if (use_p) add_mass_words(own_lo + copy, own_hi + copy, (uint32_t)bin, w);
   };
-  // The bins of all CTAs into the row's histogram, the digit that CTA 0 chooses into every CTA.  A CTA's own
-  // bins go back to zero; with `keep` the row's histogram stays for what is added to it next.
-  DigitSearch search = {0u, 0ull, 0ull};
+  // The bins of all CTAs into the row's histogram, the digit that CTA 0 chooses into every CTA, with the
+  // entries in it and whether even what lies below the first digit passes.  A CTA's own bins go back to zero;
+  // with `keep`, in that last case, the row's histogram stays for what is added to it next.
   const auto choose_in_cluster = [&](bool keep) {
     __syncthreads();
     for (int b = tid; b < FILTER_BINS; b += FILTER_THREADS) {
@@ -623,142 +750,223 @@ filter_threshold_cluster_kernel(const float* __restrict__ logits, int vocab, lon
       if (c != 0u) atomicAdd(&count0[b], c);
       if (w != 0ull) atomicAdd(&mass0[b], w);
     }
-    cluster_sync_all();
+    cluster_meet();
     if (rank == 0u) {
       const unsigned int c0 = row_count[2 * tid], c1 = row_count[2 * tid + 1];
       const unsigned long long m0 = row_mass[2 * tid], m1 = row_mass[2 * tid + 1];
       const DigitSearch before = search;
       const unsigned int digit = choose_digit(c0, c1, m0, m1, false, use_k, k, use_p, p, search, sc, sm, &choice);
+      bool all = false;
+      if (digit == 0u) {
+        if (tid == 0)
+          chosen_all = (!use_k || search.above_count + c0 < (unsigned int)k) &&
+                       (!use_p || search.above_mass + m0 < search.mass_limit);
+        __syncthreads();
+        all = chosen_all != 0u;
+      }
       if (tid == (int)(digit >> 1))
         for (unsigned int c = 0; c < CLUSTER; ++c) {
           *cluster_peer(&chosen_digit, c) = digit;
           *cluster_peer(&chosen_entries, c) = (digit & 1u) ? c1 : c0;
+          *cluster_peer(&chosen_all, c) = all;
         }
-      if (keep && digit == 0u)
+      if (keep && all)
         search = before;
       else
         row_count[2 * tid] = row_count[2 * tid + 1] = 0u, row_mass[2 * tid] = row_mass[2 * tid + 1] = 0ull;
     }
-    cluster_sync_all();
+    cluster_meet();
     return chosen_digit;
   };
 
-  // The near entries' histogram and the mass of all.
-  constexpr int NEAR_FROM = FILTER_BINS - FC_NEAR;
-  unsigned long long total = 0ull;
-  sweep_row(own_row, entries, vectors, [&](float x) {
-    const float s = __fmul_rn(x, inv_t);
-    if (!(s == s)) return;  // NaN is never a candidate
-    const int bin = distance_bin(s, top);
-    if (use_p) {
-      const unsigned long long w = fixed_mass(expf(s - top));
-      total += w;
-      if (bin >= NEAR_FROM) add_mass_words(own_lo + copy, own_hi + copy, (uint32_t)bin, w);
-    }
-    if (bin >= NEAR_FROM) atomicAdd(&own_count[copy + bin], 1u);
-  });
-  if (use_p) {
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
-    if ((tid & 31) == 0) sm[tid >> 5] = total;
-    __syncthreads();
-    if (tid < 32) {
-      total = sm[tid];
-#pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) total += __shfl_xor_sync(0xffffffffu, total, offset);
-      if (tid == 0) *cluster_peer(&peer_total[rank], 0u) = total;
-    }
-    cluster_sync_all();
-    if (rank == 0u) {
-      total = 0ull;
-#pragma unroll
-      for (int c = 0; c < CLUSTER; ++c) total += peer_total[c];
-      // (At least one: the largest entry, with nothing above it, is always a candidate.)
-      search.mass_limit = max(1ull, (unsigned long long)((double)p * (double)total));
-    }
-  }
-  unsigned int bin = choose_in_cluster(true);
-  if (bin == 0u) {  // (Everything near the maximum passes.)
-    sweep_row(own_row, entries, vectors, [&](float x) {
-      const float s = __fmul_rn(x, inv_t);
+  if (use_p && !total_first) {
+    for_each([&](float s) {
       if (!(s == s)) return;
-      const int far = distance_bin(s, top);
-      if (far < NEAR_FROM) count_entry(far, s);
+      const unsigned long long w = mass_of(s);
+      total += w;
+      if (s >= near) count_entry(bin_of(s), w);
     });
-    bin = choose_in_cluster(false);
+    share_total();
+  } else {
+    for_each([&](float s) {
+      if (s >= near) count_entry(bin_of(s), mass_of(s));
+    });
   }
-
-  const bool no_mass = use_p && total == 0ull;  // in CTA 0: a row whose maximum is not finite
-  const unsigned int in_bin = chosen_entries;
-  if (in_bin <= (unsigned int)FC_LIST) {
-    unsigned int* list0 = cluster_peer(list_key, 0u);
-    unsigned int* listed0 = cluster_peer(&listed, 0u);
-    sweep_row(own_row, entries, vectors, [&](float x) {
-      const float s = __fmul_rn(x, inv_t);
-      if (!(s == s) || distance_bin(s, top) != (int)bin) return;
-      const unsigned int at = atomicAdd(listed0, 1u);
-      if (at < (unsigned int)FC_LIST) list0[at] = float_key(s);
+  unsigned int bin = choose_in_cluster(near > lowest);
+  float next = use_p ? fmaxf(lowest, reach()) : lowest;
+  while (chosen_all != 0u && near > lowest) {  // (The threshold is not among the entries so far.)
+    const float until = near;
+    near = next < until ? next : lowest;
+    next = lowest;
+    for_each([&](float s) {
+      if (s >= near && s < until) count_entry(bin_of(s), mass_of(s));
     });
-    cluster_sync_all();
-    if (rank != 0u) return;
-    const bool mine = tid < (int)in_bin;
-    const uint32_t key = mine ? list_key[tid] : 0u;
-    if (mine) list_mass[tid] = use_p ? fixed_mass(expf(key_float(key) - top)) : 0ull;
-    __syncthreads();
-    unsigned int above = search.above_count;
-    unsigned long long mass = search.above_mass;
-    if (mine)
-      for (int j = 0; j < (int)in_bin; ++j)
-        if (list_key[j] > key) above += 1u, mass += list_mass[j];
-    const bool passes = mine && (!use_k || above < (unsigned int)k) && (!use_p || mass < search.mass_limit);
-    const unsigned int smallest = __reduce_min_sync(0xffffffffu, passes ? key : 0xffffffffu);
-    if ((tid & 31) == 0) sc[tid >> 5] = smallest;
-    // Bin 0 and every entry passes: no value is too small (a row with NaN that has fewer than k entries).
-    unsigned long long bin_mass = mine && use_p ? list_mass[tid] : 0ull;
-#pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) bin_mass += __shfl_xor_sync(0xffffffffu, bin_mass, offset);
-    if ((tid & 31) == 0) sm[tid >> 5] = bin_mass;
-    __syncthreads();
-    if (tid < 32) {
-      const unsigned int found = __reduce_min_sync(0xffffffffu, sc[tid]);
-      bin_mass = sm[tid];
-#pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) bin_mass += __shfl_xor_sync(0xffffffffu, bin_mass, offset);
-      const bool all = bin == 0u && (!use_k || search.above_count + in_bin < (unsigned int)k) &&
-                       (!use_p || search.above_mass + bin_mass < search.mass_limit);
-      if (tid == 0) threshold[r] = no_mass ? top : all ? key_float(0u) : key_float(found);
-    }
+    bin = choose_in_cluster(near > lowest);
+  }
+  if (chosen_all != 0u) {  // No value is too small: a row with NaN that has fewer than k entries.
+    if (rank == 0u && tid == 0) threshold[r] = key_float(0u);
     return;
   }
 
-  // Too many for a list: digit by digit over the entries of the bin.
-  uint32_t prefix = 0u;
-  const int shifts[3] = {21, 10, 0};
-  const int bits[3] = {11, 11, 10};
-#pragma unroll
-  for (int level = 0; level < 3; ++level) {
-    const int shift = shifts[level], level_bits = bits[level];
-    const uint32_t digit_mask = (1u << level_bits) - 1u;
-    sweep_row(own_row, entries, vectors, [&](float x) {
-      const float s = __fmul_rn(x, inv_t);
-      if (!(s == s) || distance_bin(s, top) != (int)bin) return;
+  // The patterns of the bin's entries: all of them, or, of more than FC_LIST, the range that holds the threshold.
+  uint32_t lo = 0u, hi = 0xffffffffu;
+  if (chosen_entries > (unsigned int)FC_LIST) {
+    uint32_t least_key = 0xffffffffu, most_key = 0u;
+    for_each([&](float s) {
+      if (!(s >= near) || bin_of(s) != (int)bin) return;
       const uint32_t key = float_key(s);
-      if (level > 0 && (key >> (shift + level_bits)) != prefix) return;
-      count_entry((int)((key >> shift) & digit_mask), s);
+      least_key = min(least_key, key), most_key = max(most_key, key);
     });
-    prefix = (prefix << level_bits) | choose_in_cluster(false);
+    least_key = __reduce_min_sync(0xffffffffu, least_key), most_key = __reduce_max_sync(0xffffffffu, most_key);
+    if (lane == 0) sc[warp] = least_key, sm[warp] = most_key;
+    __syncthreads();
+    if (tid < 32) {
+      const uint2 mine = make_uint2(__reduce_min_sync(0xffffffffu, sc[tid]), __reduce_max_sync(0xffffffffu, (uint32_t)sm[tid]));
+      if (tid < CLUSTER) *cluster_peer(&peer_range[rank], (unsigned int)tid) = mine;
+    }
+    cluster_meet();
+    lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+    for (int c = 0; c < CLUSTER; ++c) lo = min(lo, peer_range[c].x), hi = max(hi, peer_range[c].y);
+    while (lo < hi && chosen_entries > (unsigned int)FC_LIST) {
+      const int shift = pattern_shift(lo, hi);
+      for_each([&](float s) {
+        if (!(s >= near) || bin_of(s) != (int)bin) return;
+        const uint32_t key = float_key(s);
+        if (key >= lo && key <= hi) count_entry((int)((key - lo) >> shift), mass_of(s));
+      });
+      lo += choose_in_cluster(false) << shift;
+      hi = min(hi, lo + ((1u << shift) - 1u));
+    }
+    if (lo == hi) {
+      if (rank == 0u && tid == 0) threshold[r] = key_float(lo);
+      return;
+    }
   }
-  if (rank == 0u && tid == 0) threshold[r] = no_mass ? top : key_float(prefix);
+  unsigned int* list0 = cluster_peer(list_key, 0u);
+  unsigned int* listed0 = cluster_peer(&listed, 0u);
+  for_each([&](float s) {
+    if (!(s >= near) || bin_of(s) != (int)bin) return;
+    const uint32_t key = float_key(s);
+    if (key < lo || key > hi) return;
+    const unsigned int together = __activemask();  // one request of the lanes that are here
+    unsigned int at = 0u;
+    if (lane == __ffs(together) - 1) at = atomicAdd(listed0, __popc(together));
+    at = __shfl_sync(together, at, __ffs(together) - 1) + __popc(together & ((1u << lane) - 1u));
+    if (at < (unsigned int)FC_LIST) list0[at] = key;
+  });
+  cluster_meet();
+  if (rank != 0u) return;
+
+  // CTA 0 alone: an entry a thread.  More than can be compared with one another are narrowed first.
+  int n = (int)chosen_entries;
+  bool mine = tid < n;
+  const uint32_t key = mine ? list_key[tid] : 0u;
+  const unsigned long long mass = mine ? mass_of(key_float(key)) : 0ull;
+  if (n > FC_PAIRS) {
+    while (true) {
+      const uint32_t least_key = __reduce_min_sync(0xffffffffu, mine ? key : 0xffffffffu);
+      const uint32_t most_key = __reduce_max_sync(0xffffffffu, mine ? key : 0u);
+      if (lane == 0) sc[warp] = least_key, sm[warp] = most_key;
+      __syncthreads();
+      lo = __reduce_min_sync(0xffffffffu, sc[lane]), hi = __reduce_max_sync(0xffffffffu, (uint32_t)sm[lane]);
+      if (n <= FC_PAIRS || lo == hi) break;
+      const int shift = pattern_shift(lo, hi);
+      if (mine) {
+        atomicAdd(&own_count[(key - lo) >> shift], 1u);
+        if (use_p) add_mass_words(own_lo, own_hi, (key - lo) >> shift, mass);
+      }
+      __syncthreads();
+      const int at = 2 * tid;
+      const unsigned int c0 = own_count[at], c1 = own_count[at + 1];
+      const unsigned long long m0 = ((unsigned long long)own_hi[at] << 32) + own_lo[at];
+      const unsigned long long m1 = ((unsigned long long)own_hi[at + 1] << 32) + own_lo[at + 1];
+      own_count[at] = own_count[at + 1] = own_lo[at] = own_lo[at + 1] = own_hi[at] = own_hi[at + 1] = 0u;
+      lo += choose_digit(c0, c1, m0, m1, false, use_k, k, use_p, p, search, sc, sm, &choice) << shift;
+      hi = min(hi, lo + ((1u << shift) - 1u));
+      mine = mine && key >= lo && key <= hi;
+      n = __syncthreads_count(mine);
+    }
+    if (lo == hi) {
+      if (tid == 0) threshold[r] = key_float(lo);
+      return;
+    }
+    if (tid == 0) listed = 0u;
+  }
+  __syncthreads();
+  if (n < (int)chosen_entries) {
+    if (mine) {
+      const unsigned int at = atomicAdd(&listed, 1u);
+      list_key[at] = key, list_mass[at] = mass;
+    }
+  } else if (mine) {
+    list_mass[tid] = mass;
+  }
+  __syncthreads();
+  unsigned int above = search.above_count;
+  unsigned long long above_mass = search.above_mass;
+  if (mine) {
+#pragma unroll 4
+    for (int j = 0; j < n; ++j)
+      if (list_key[j] > key) above += 1u, above_mass += list_mass[j];
+  }
+  const bool passes = mine && (!use_k || above < (unsigned int)k) && (!use_p || above_mass < search.mass_limit);
+  const unsigned int smallest = __reduce_min_sync(0xffffffffu, passes ? key : 0xffffffffu);
+  if (lane == 0) sc[warp] = smallest;
+  __syncthreads();
+  if (tid < 32) {
+    const unsigned int found = __reduce_min_sync(0xffffffffu, sc[tid]);
+    if (tid == 0) threshold[r] = key_float(found);
+  }
+}
+
+// In a cluster of eight, a CTA's share of the longest row fits its shared memory.
+template <int CLUSTER>
+constexpr auto filter_cluster = filter_threshold_cluster_kernel<CLUSTER, CLUSTER == 8>;
+template <int CLUSTER>
+constexpr size_t filter_cluster_smem = FC_SMEM_BYTES + (CLUSTER == 8 ? FC_SHARE * sizeof(float) : 0);
+
+template <int CLUSTER>
+cudaError_t allow_filter_cluster() {
+  static const cudaError_t ready = cudaFuncSetAttribute(filter_cluster<CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                        (int)filter_cluster_smem<CLUSTER>);
+  return ready;
+}
+
+// Rows that the device works on at once with this many CTAs a row.  (A CTA fills an SM, and whole clusters
+// lie in a GPC: on 148 SMs there is room for 16 clusters of eight, not 18.)
+template <int CLUSTER>
+int filter_rows_at_once() {
+  static const int rows = [] {
+    if (allow_filter_cluster<CLUSTER>() != cudaSuccess) return 0;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(CLUSTER * 64);
+    config.blockDim = dim3(FILTER_THREADS);
+    config.dynamicSmemBytes = filter_cluster_smem<CLUSTER>;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = CLUSTER;
+    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, filter_cluster<CLUSTER>, &config) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return clusters;
+  }();
+  return rows;
 }
 
 template <int CLUSTER>
 cudaError_t launch_filter_cluster(const float* logits, int num_rows, int vocab, long long row_stride, const float* temperature,
                                   const int* top_k, const float* top_p, float* threshold, cudaStream_t stream) {
-  static const cudaError_t ready = cudaFuncSetAttribute(filter_threshold_cluster_kernel<CLUSTER>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FC_SMEM_BYTES);
+  const cudaError_t ready = allow_filter_cluster<CLUSTER>();
   if (ready != cudaSuccess) return ready;
-  return launch_pdl_cluster(filter_threshold_cluster_kernel<CLUSTER>, dim3((unsigned)num_rows * CLUSTER), dim3(FILTER_THREADS),
-                            FC_SMEM_BYTES, CLUSTER, stream, logits, vocab, row_stride, temperature, top_k, top_p, threshold);
+  return launch_pdl_cluster(filter_cluster<CLUSTER>, dim3((unsigned)num_rows * CLUSTER), dim3(FILTER_THREADS),
+                            filter_cluster_smem<CLUSTER>, CLUSTER, stream, logits, vocab, row_stride, temperature, top_k, top_p,
+                            threshold);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -838,7 +1046,7 @@ VX_API int vx_sample(const float* logits, int num_rows, int vocab, long long row
   return (int)cudaGetLastError();
 }
 
-// kind 0: the cluster kernel where the row fits its registers, else one CTA a row; 1: one CTA a
+// kind 0: the cluster kernel for rows of up to 196,608 entries, else one CTA a row; 1: one CTA a
 // row; 2: the cluster kernel or an error.
 VX_API int vx_filter_threshold(const float* logits, int num_rows, int vocab, long long row_stride,
                                const float* temperature, const int* top_k, const float* top_p,
@@ -853,9 +1061,9 @@ VX_API int vx_filter_threshold(const float* logits, int num_rows, int vocab, lon
   }
   if (kind == 2 && vocab > FC_MAX_VOCAB) return (int)cudaErrorInvalidValue;
   if (kind != 1 && vocab <= FC_MAX_VOCAB) {
-    // A CTA fills an SM: the largest cluster with which all rows run at once.
-    const auto launch = num_rows * 8 <= 144 ? launch_filter_cluster<8>
-                        : num_rows * 4 <= 144 ? launch_filter_cluster<4> : launch_filter_cluster<2>;
+    // The largest cluster with which all rows run at once.
+    const auto launch = num_rows <= filter_rows_at_once<8>() ? launch_filter_cluster<8>
+                        : num_rows <= filter_rows_at_once<4>() ? launch_filter_cluster<4> : launch_filter_cluster<2>;
     return (int)launch(logits, num_rows, vocab, row_stride, temperature, top_k, top_p, threshold, stream);
   }
   launch_pdl(filter_threshold_kernel, dim3(num_rows), dim3(FILTER_THREADS), FILTER_SMEM_BYTES, stream, logits, vocab, row_stride,
