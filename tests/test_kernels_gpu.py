@@ -203,6 +203,20 @@ def test_add_rmsnorm_many_wide_rows(k, hidden, T):
     check_add_rmsnorm(k, torch.bfloat16, hidden, T)
 
 
+@pytest.mark.parametrize("hidden", [4100, 5120, 5124, 7000, 8192])
+def test_add_rmsnorm_wide_rows_do_not_depend_on_the_step(k, hidden):
+    """Rows of more than 4,096 elements have the same bits in a step of many rows and in one of few."""
+    gen = torch.Generator().manual_seed(hidden)
+    resid = (torch.randn(704, hidden, generator=gen) * 3).cuda()
+    delta = torch.randn(704, hidden, generator=gen).to(torch.bfloat16).cuda()
+    weight = (1 + 0.1 * torch.randn(hidden, generator=gen)).cuda()
+    out, few = (torch.empty(704, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for i in range(0, 704, 176):
+        k.add_rmsnorm(resid[i : i + 176].clone(), delta[i : i + 176], weight, 1e-6, few[i : i + 176], 176)
+    k.add_rmsnorm(resid, delta, weight, 1e-6, out, 704)
+    assert torch.equal(out, few)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("hidden,T", [(1536, 700), (3584, 300), (240, 513), (4100, 260)])
 def test_add_rmsnorm_many_rows(k, dtype, hidden, T):

@@ -552,19 +552,24 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __res
 // The same with a few warps per row, for steps of many rows: a lane keeps its share of the row
 // (chunks idx, idx + lanes, ... of four elements) in registers and has all its loads under way
 // at once, the sum of squares goes through shuffles and one exchange between the row's warps,
-// and a block (two rows) meets once between its loads and its stores.  (One block per row reached
-// about half of the memory bandwidth at 2,048 rows: three waves of blocks that each load, meet,
-// and store.)
-template <typename T, int MAX_CHUNKS, int WPR>
+// and a block (two rows of four warps, one of eight) meets once between its loads and its stores.
+// (One block per row reached about half of the memory bandwidth at 2,048 rows: three waves of
+// blocks that each load, meet, and store.)
+//
+// SUMS 3 and 4 (eight warps, rows of more than 4,096 elements): a lane makes the sums of that many
+// threads of the kernel above, two chunks each, and they are added up in that kernel's order, so a
+// row has the same bits in either.
+template <typename T, int MAX_CHUNKS, int WPR, int SUMS>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ weight,
                         float eps, T* __restrict__ out, const int* __restrict__ rows, int hidden, int write_resid,
-                        int num_rows) {
+                        int num_rows, int block) {
   // WPR warps share a row (their 32 * WPR lanes take chunks idx, idx + 32 * WPR, ...):
   // fewer instructions per warp, whose chain is what a launch of one wave takes, and the weights
   // are asked for together with the row, not after the sum.
   constexpr int LANES = 32 * WPR;
-  __shared__ float warp_sums[8];
+  __shared__ float warp_sums[8 * SUMS];
+  static_assert(SUMS == 1 || (WPR == 8 && SUMS <= 4 && MAX_CHUNKS == 2 * SUMS), "two chunks for each thread of a block");
   VX_TRACE_SCOPE(2);
   allow_dependents();
   grid_dependency_wait();
@@ -574,19 +579,25 @@ add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, 
   const bool live = o < num_rows;
   const int r = live ? (rows ? rows[o] : o) : 0;
   const int chunks = live ? hidden >> 2 : 0;
+  // This lane's chunks; with several sums, those of thread idx + 256 i of a block of `block` threads.
+  const auto chunk_at = [&](int j) {
+    if constexpr (SUMS == 1) return idx + LANES * j;
+    const int thread = idx + LANES * (j % SUMS);
+    return thread >= block ? chunks : j < SUMS ? thread : thread + block;
+  };
   float* x = resid + (size_t)r * hidden;
   const T* d = delta ? delta + (size_t)r * hidden : nullptr;
   float4 vals[MAX_CHUNKS], w[MAX_CHUNKS];
-  float ss = 0.f;
+  float part[SUMS], ss = 0.f;
 #pragma unroll
   for (int j = 0; j < MAX_CHUNKS; ++j) {
-    const int c = idx + LANES * j;
+    const int c = chunk_at(j);
     vals[j] = c < chunks ? *reinterpret_cast<const float4*>(x + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (d) {
 #pragma unroll
     for (int j = 0; j < MAX_CHUNKS; ++j) {
-      const int c = idx + LANES * j;
+      const int c = chunk_at(j);
       if (c < chunks) {
         const float4 e = load4_as_float<T>(d + 4 * c);
         vals[j].x += e.x;
@@ -598,25 +609,33 @@ add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, 
   }
 #pragma unroll
   for (int j = 0; j < MAX_CHUNKS; ++j) {
-    const int c = idx + LANES * j;
+    const int c = chunk_at(j);
     w[j] = c < chunks ? __ldg(reinterpret_cast<const float4*>(weight + 4 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
+  for (int i = 0; i < SUMS; ++i) part[i] = 0.f;
+#pragma unroll
   for (int j = 0; j < MAX_CHUNKS; ++j)
-    ss += vals[j].x * vals[j].x + vals[j].y * vals[j].y + vals[j].z * vals[j].z + vals[j].w * vals[j].w;
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) warp_sums[warp] = ss;
+    part[j % SUMS] += vals[j].x * vals[j].x + vals[j].y * vals[j].y + vals[j].z * vals[j].z + vals[j].w * vals[j].w;
+#pragma unroll
+  for (int i = 0; i < SUMS; ++i) {
+    part[i] = warp_sum(part[i]);
+    if ((threadIdx.x & 31) == 0) warp_sums[i * 8 + warp] = part[i];
+  }
   __syncthreads();
   if (!live) return;
   // The same terms in the same order in every warp of the row.
-  ss = 0.f;
+  if constexpr (SUMS == 1) {
 #pragma unroll
-  for (int i = 0; i < WPR; ++i) ss += warp_sums[(warp / WPR) * WPR + i];
+    for (int i = 0; i < WPR; ++i) ss += warp_sums[(warp / WPR) * WPR + i];
+  } else {
+    ss = warp_sum((threadIdx.x & 31) < 8 * SUMS ? warp_sums[threadIdx.x & 31] : 0.f);
+  }
   const float inv = 1.0f / sqrtf(ss / (float)hidden + eps);
   T* y = out + (size_t)o * hidden;
 #pragma unroll
   for (int j = 0; j < MAX_CHUNKS; ++j) {
-    const int c = idx + LANES * j;
+    const int c = chunk_at(j);
     if (c < chunks) {
       const float4 v = vals[j];
       if (write_resid && d) *reinterpret_cast<float4*>(x + 4 * c) = v;
@@ -626,13 +645,20 @@ add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, 
   }
 }
 
-template <typename T, int MAX_CHUNKS, int WPR>
+// Threads of a block that has a row: a chunk of four elements each, two in rows of more than 4,096 elements.
+static int norm_block(int hidden) {
+  const int chunks = hidden / 4;
+  const int block = ((chunks <= 1024 ? chunks : (chunks + 1) / 2) + 31) / 32 * 32;
+  return block < 64 ? 64 : block;
+}
+
+template <typename T, int MAX_CHUNKS, int WPR, int SUMS = 1>
 static void launch_rmsnorm_warp(float* resid, const void* delta, const float* weight, float eps, void* out,
                                 const int* rows, int num_rows, int hidden, int write_resid, cudaStream_t stream) {
   const int rows_per_block = 8 / WPR;  // eight warps
-  launch_pdl(add_rmsnorm_warp_kernel<T, MAX_CHUNKS, WPR>, dim3((num_rows + rows_per_block - 1) / rows_per_block),
+  launch_pdl(add_rmsnorm_warp_kernel<T, MAX_CHUNKS, WPR, SUMS>, dim3((num_rows + rows_per_block - 1) / rows_per_block),
              dim3(256), 0, stream, resid, (const T*)delta, weight, eps, (T*)out, rows, hidden, write_resid,
-             num_rows);
+             num_rows, norm_block(hidden));
 }
 
 VX_API int vx_add_rmsnorm(float* resid, const void* delta, const float* weight, float eps,
@@ -644,23 +670,22 @@ VX_API int vx_add_rmsnorm(float* resid, const void* delta, const float* weight, 
   // Many rows: a few warps per row (rows of up to 8,192 elements, whole chunks of four).  Not in
   // the float32 path: there a row's sum of squares is added up in the same order whatever the
   // step, so that results do not depend on how the work was cut.
-  if (aligned && dtype == VX_DTYPE_BF16 && num_out_rows >= 256 && hidden % 4 == 0 && hidden <= 8192) {
+  // From 256 rows on; between 4,096 and 6,144 elements from 297, since up to two rows an SM a block a row is
+  // one wave and no slower (5,120 elements: 256 rows 5.0 us against 5.2, 296 rows 5.2 against 5.4, 297 rows 6.8 against 5.4).
+  const int many_rows = hidden > 4096 && hidden <= 6144 ? 297 : 256;
+  if (aligned && dtype == VX_DTYPE_BF16 && num_out_rows >= many_rows && hidden % 4 == 0 && hidden <= 8192) {
     // Four warps a row (measured in a prefill of the 1.5B sizes: 9.1 us a launch at 2,048 rows
     // with one warp a row, 7.9 with two, 6.8 with four, 7.3 with eight; 8.5 -> 3.1 us at 512 rows).
     if (hidden <= 2048) launch_rmsnorm_warp<__nv_bfloat16, 4, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
     else if (hidden <= 4096) launch_rmsnorm_warp<__nv_bfloat16, 8, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
-    // Eight warps a row beyond that, five chunks a lane at 5,120 elements (a block of 1,024 threads a row before:
-    // 28.6 us a launch at 2,048 rows; the 14B sizes' portion of 2,048 tokens 71.9 -> 71.3 ms).
-    else if (hidden <= 5120) launch_rmsnorm_warp<__nv_bfloat16, 5, 8>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
-    else launch_rmsnorm_warp<__nv_bfloat16, 8, 8>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
+    // Eight warps a row beyond that (2,048 rows, out of memory: 5,120 elements 29.3 -> 20.3 us, 8,192 55.2 -> 34.4;
+    // with a sum a lane, other bits, 20.2 and 34.1).
+    else if (hidden <= 6144) launch_rmsnorm_warp<__nv_bfloat16, 6, 8, 3>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
+    else launch_rmsnorm_warp<__nv_bfloat16, 8, 8, 4>(resid, delta, weight, eps, out, rows, num_out_rows, hidden, write_resid, stream);
     return (int)cudaGetLastError();
   }
   if (aligned && hidden % 4 == 0 && hidden / 4 <= 1024 * NORM_VEC_CHUNKS) {
-    // One chunk of four per thread, two for rows of more than 4,096 elements.
-    const int chunks = hidden / 4;
-    int block = chunks <= 1024 ? chunks : (chunks + 1) / 2;
-    block = (block + 31) / 32 * 32;
-    if (block < 64) block = 64;
+    const int block = norm_block(hidden);
     if (dtype == VX_DTYPE_F32)
       launch_pdl(add_rmsnorm_vec_kernel<float>, dim3(num_out_rows), dim3(block), 0, stream, resid,
                  (const float*)delta, weight, eps, (float*)out, rows, hidden, write_resid);
