@@ -269,7 +269,7 @@ def plain_paged_attention(q, k_all, v_all, ctx, scale, window):
 
 def run_attention_case(k, dtype, H, G, D, P, seqs, window=None, seed=0, min_split_keys=256,
                        target_ctas=296, spike=None, fused_merge=True, max_cluster=1, max_splits=64,
-                       tensor_memory=False, ramp=None, tc_ctas_per_sm=1, tc_merge_us=30.0, spike_scale=12, cache_offset=0):
+                       tensor_memory=False, ramp=None, tc_ctas_per_sm=1, tc_merge_us=30.0, cache_offset=0):
     """seqs: list of (q_len, ctx_len).  Returns (got, want) as float64 [T, H, D]."""
     from velox_b200.ops import attention_plan as ap
 
@@ -297,9 +297,9 @@ def run_attention_case(k, dtype, H, G, D, P, seqs, window=None, seed=0, min_spli
             page, off = pages[key_index // P], key_index % P
             direction = torch.randn(D, generator=gen)
             direction = direction / direction.norm()
-            k_cache[page, off, :, :] = (direction * spike_scale).to(dtype)
+            k_cache[page, off, :, :] = (direction * 12).to(dtype)
             q_view = qkv[row + qi, : H * D].view(H, D)
-            q_view[:] = (direction * spike_scale).to(dtype)
+            q_view[:] = (direction * 12).to(dtype)
         slots = [pages[i // P] * P + i % P for i in range(kv_len)]
         if ramp is not None:
             # Every query looks along one direction and the keys' share of it grows with the
