@@ -423,6 +423,19 @@ def test_attention_cluster_shares_an_item(k, H, G, D, P, max_cluster, max_splits
 
 
 # One CTA per SM with P in shared memory over the K tile, or two with P in tensor memory.
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("D", [16, 128, 256])
+def test_attention_merge_of_many_splits(k, dtype, D):
+    """Key ranges split more than sixteen, thirty-two and forty-eight times (a batch of loads, a lane's first
+    weight), the last batch not full, through the merge kernel."""
+    got, want, plan = run_attention_case(k, dtype, 6, 2, D, 16, [(1, 1099), (1, 2399), (3, 4150), (2, 3300)], seed=D,
+                                         min_split_keys=64, target_ctas=2000, fused_merge=False)
+    splits = sorted(int(item[4]) for item in plan.merge_items)
+    assert splits[0] > 16 and splits[-1] > 48 and any(s > 32 and s % 16 for s in splits), splits
+    err = (got - want).abs().max().item()
+    assert err <= _attn_tol(dtype) * want.abs().max().item(), err
+
+
 TC_FORMS = pytest.mark.parametrize("per_sm", [1, 2], ids=["p_in_shared_memory", "p_in_tensor_memory"])
 
 

@@ -57,8 +57,7 @@
 namespace vx {
 
 constexpr int D = VX_HEAD_DIM;
-// A key range is cut into at most this many splits (the merge kernel keeps their weights in
-// shared memory).
+// A key range is cut into at most this many splits (a lane of the merge kernel has the weights of two).
 constexpr int ATTN_MAX_SPLITS = 64;
 
 struct AttnArgs {
@@ -690,13 +689,14 @@ __device__ __forceinline__ void store_rows(const AttnArgs& a, const float (&o)[D
 //   {seq, row_begin, row_count, first_partial_base, num_splits, split_stride, -, -}
 // split s of the item wrote its rows at first_partial_base + s * split_stride.
 // A warp merges a row: lane s has the weights of splits s and s + 32, every lane four neighbouring dims of
-// the row, all splits' loads under way together.  (A block per row, with two barriers between its loads,
+// the row, the loads of BATCH splits under way together and the first of them before the weights' own.
+// (A block per row, with two barriers between its loads,
 // was four waves of blocks that each waited for one load after the other: 34 us for the 500-token portion
 // of a sixteen-head layer with a sink; a step of the Mamivik 0.5b sizes with such a portion, replayed, 4.39 -> 4.32 ms.)
 // =============================================================================================
 constexpr int MERGE_WARPS = 8;
 
-template <typename T>
+template <typename T, int BATCH>
 __global__ void __launch_bounds__(32 * MERGE_WARPS) attn_merge_kernel(AttnArgs a, const int* __restrict__ merge_items) {
   VX_TRACE_SCOPE(22);
   allow_dependents();
@@ -712,6 +712,27 @@ __global__ void __launch_bounds__(32 * MERGE_WARPS) attn_merge_kernel(AttnArgs a
   const int tok = row / a.group, hg = row - tok * a.group;
   const int head = kvh * a.group + hg;
   static_assert(ATTN_MAX_SPLITS <= 64, "a lane has the weights of two splits");
+  const bool vec_in = ((uintptr_t)a.partial_o & 15) == 0;
+  float4 part[BATCH];
+  // Asks for this lane's dims, d ... d + 3, of the splits from s0 on, four splits at a time.
+  const auto request = [&](int d, int s0) {
+#pragma unroll
+    for (int g = 0; g < BATCH; g += 4) {
+      if (s0 + g >= splits) continue;
+#pragma unroll
+      for (int i = g; i < g + 4; ++i) {
+        // (With sixteen the last splits and the row's last dims are asked for again rather than branched over:
+        // 64 splits 5.8 us a launch against 7.7; with four that costs more than the branch.)
+        if (BATCH == 4 && s0 + i >= splits) continue;
+        const float* from = a.partial_o + (base + (size_t)min(s0 + i, splits - 1) * stride) * D + min(d, D - 4);
+        if (vec_in)
+          part[i] = __ldcg(reinterpret_cast<const float4*>(from));
+        else
+          part[i] = make_float4(__ldcg(from), __ldcg(from + 1), __ldcg(from + 2), __ldcg(from + 3));
+      }
+    }
+  };
+  request(lane * 4, 0);
   const float lse0 = lane < splits ? __ldcg(&a.partial_lse[base + (size_t)lane * stride]) : -CUDART_INF_F;
   const float lse1 = lane + 32 < splits ? __ldcg(&a.partial_lse[base + (size_t)(lane + 32) * stride]) : -CUDART_INF_F;
   float mt = warp_max(fmaxf(lse0, lse1));
@@ -727,24 +748,27 @@ __global__ void __launch_bounds__(32 * MERGE_WARPS) attn_merge_kernel(AttnArgs a
   float den = warp_sum(w0 + w1);
   if (sink != -CUDART_INF_F) den += exp2f(sink - m_safe);
   T* dst = (T*)a.out + (size_t)(a.q_start[seq] + tok) * a.out_stride + (size_t)head * D;
-  const bool vec = ((uintptr_t)dst & (sizeof(T) * 4 - 1)) == 0, vec_in = ((uintptr_t)a.partial_o & 15) == 0;
+  const bool vec = ((uintptr_t)dst & (sizeof(T) * 4 - 1)) == 0;
 #pragma unroll
   for (int d0 = 0; d0 < D; d0 += 128) {
     const int d = d0 + lane * 4;
     const bool on = d < D;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int s = 0; s < splits; ++s) {
-      const float w = __shfl_sync(0xffffffffu, s < 32 ? w0 : w1, s & 31);
-      const float* from = a.partial_o + (base + (size_t)s * stride) * D + d;
-      float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (on)
-        o = vec_in ? __ldcg(reinterpret_cast<const float4*>(from))
-                   : make_float4(__ldcg(from), __ldcg(from + 1), __ldcg(from + 2), __ldcg(from + 3));
-      acc[0] += w * o.x;
-      acc[1] += w * o.y;
-      acc[2] += w * o.z;
-      acc[3] += w * o.w;
+    for (int s0 = 0; s0 < splits; s0 += BATCH) {
+      if (d0 + s0 > 0) request(d, s0);
+#pragma unroll
+      for (int g = 0; g < BATCH; g += 4) {
+        if (s0 + g >= splits) continue;
+#pragma unroll
+        for (int i = g; i < g + 4; ++i) {
+          if (s0 + i >= splits) continue;
+          const float w = __shfl_sync(0xffffffffu, s0 < 32 ? w0 : w1, (s0 + i) & 31);
+          acc[0] += w * part[i].x;
+          acc[1] += w * part[i].y;
+          acc[2] += w * part[i].z;
+          acc[3] += w * part[i].w;
+        }
+      }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = den > 0.f ? acc[i] / den : 0.f;
@@ -2707,11 +2731,17 @@ VX_API int vx_attention_merge(int dtype, void* out, const int* q_start, const in
                          merge_items, nullptr, 0, out_stride, 0, num_kv_heads, group, 1, 0, 1.0f);
   a.sinks = sinks;
   const dim3 grid(num_items, num_kv_heads, (max_rows + MERGE_WARPS - 1) / MERGE_WARPS);
-  const int threads = 32 * MERGE_WARPS;
+  // Up to two blocks an SM: sixteen splits at a time, since the chain of loads is all there is (us a launch, heads of
+  // 128: four tokens of twelve heads in 64 splits 13.6 -> 5.8, eight of fourteen in 16 splits 4.8 -> 2.8; a block a
+  // row, before, took 6.1 and 3.4).  More blocks hide one another's loads, and as many as the registers for four
+  // splits allow do best (2,048 tokens of sixteen heads in two splits 10.9 us, with sixteen 20.6; a block a row 36).
+  const bool few = (long long)grid.x * grid.y * grid.z <= 296;
+  const dim3 block(32 * MERGE_WARPS);
   if (dtype == VX_DTYPE_F32)
-    launch_pdl(attn_merge_kernel<float>, dim3(grid), dim3(threads), 0, stream, a, merge_items);
+    launch_pdl(few ? attn_merge_kernel<float, 16> : attn_merge_kernel<float, 4>, grid, block, 0, stream, a, merge_items);
   else
-    launch_pdl(attn_merge_kernel<__nv_bfloat16>, dim3(grid), dim3(threads), 0, stream, a, merge_items);
+    launch_pdl(few ? attn_merge_kernel<__nv_bfloat16, 16> : attn_merge_kernel<__nv_bfloat16, 4>, grid, block, 0, stream, a,
+               merge_items);
   return (int)cudaGetLastError();
 }
 
