@@ -197,6 +197,17 @@ def test_gemm_f32_every_tile_sums_alike(k, N, K, offset):
         assert torch.all(out[M] == 5.0)
 
 
+def test_gemm_f32_more_weight_rows_than_a_grid_has_in_y(k):
+    """65,535 tiles of 64 weight rows and one more."""
+    N = 65535 * 64 + 5
+    a = torch.tensor([[1.0, 2.0, -3.0, 4.0]]).cuda()
+    w = torch.randn(N, 4, device="cuda")
+    out = torch.empty(1, N, device="cuda")
+    k.gemm_f32(a, w, None, out, 1)
+    want = (w.double() @ a[0].double())[None]
+    assert (out.double() - want).abs().max().item() <= 1e-5 * want.abs().max().item()
+
+
 @pytest.mark.parametrize("hidden,T", [(5120, 300), (5124, 256), (8192, 257), (8196, 256)])
 def test_add_rmsnorm_many_wide_rows(k, hidden, T):
     """Eight warps a row up to 8,192 elements, and the rows beyond."""

@@ -73,10 +73,11 @@ struct F32Tile {
   static constexpr size_t SMEM = sizeof(float) * (STAGES * STAGE_FLOATS > BM * SUM_PITCH ? STAGES * STAGE_FLOATS : BM * SUM_PITCH);
 };
 
-template <typename S>
+// ROW: C's rows are that long rather than N (a launch that makes some of the columns).
+template <typename S, bool ROW>
 __global__ void __launch_bounds__(S::THREADS, 2)
 gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                float* __restrict__ C, int M, int N, int K, int ranks, int blocks_per_rank) {
+                float* __restrict__ C, int M, int N, int K, int ranks, int blocks_per_rank, int row) {
   allow_dependents();
   extern __shared__ __align__(16) float f32_smem[];
   constexpr int TM = S::thread_m, TN = S::thread_n, STAGES = S::STAGES;
@@ -163,7 +164,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
         const int m = m0 + row_m + i * STEP_M;
-        if (m < M) C[(size_t)m * N + n] = sum_of(i, j) + add;
+        if (m < M) C[(size_t)m * (ROW ? row : N) + n] = sum_of(i, j) + add;
       }
     }
     return;
@@ -208,16 +209,32 @@ inline int f32_ranks(int N, int K) {
 template <typename S>
 int launch_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
   static const cudaError_t ready =
-      cudaFuncSetAttribute(gemm_f32_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+      cudaFuncSetAttribute(gemm_f32_kernel<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
   if (ready != cudaSuccess) return (int)ready;
   const int ranks = f32_ranks(N, K);
   const int blocks = (K + F32_BK - 1) / F32_BK;
   const dim3 grid(ranks, (N + S::BN - 1) / S::BN, (M + S::BM - 1) / S::BM);
   if (ranks == 1)
-    launch_pdl(gemm_f32_kernel<S>, grid, dim3(S::THREADS), S::SMEM, stream, A, W, bias, C, M, N, K, ranks, blocks);
+    launch_pdl(gemm_f32_kernel<S, false>, grid, dim3(S::THREADS), S::SMEM, stream, A, W, bias, C, M, N, K, ranks, blocks, N);
   else
-    launch_pdl_cluster(gemm_f32_kernel<S>, grid, dim3(S::THREADS), S::SMEM, ranks, stream, A, W, bias, C, M, N, K, ranks,
-                       (blocks + ranks - 1) / ranks);
+    launch_pdl_cluster(gemm_f32_kernel<S, false>, grid, dim3(S::THREADS), S::SMEM, ranks, stream, A, W, bias, C, M, N, K, ranks,
+                       (blocks + ranks - 1) / ranks, N);
+  return (int)cudaGetLastError();
+}
+
+// More weight rows than a grid has tiles in y, 65,535 of 64: one launch after the other.
+template <typename S>
+int launch_gemm_f32_parts(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t stream) {
+  static const cudaError_t ready =
+      cudaFuncSetAttribute(gemm_f32_kernel<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+  if (ready != cudaSuccess) return (int)ready;
+  const int blocks = (K + F32_BK - 1) / F32_BK;
+  constexpr int MOST = 65535 * S::BN;
+  for (long long n = 0; n < N; n += MOST) {
+    const int part = (int)(N - n < MOST ? N - n : MOST);
+    launch_pdl(gemm_f32_kernel<S, true>, dim3(1, (part + S::BN - 1) / S::BN, (M + S::BM - 1) / S::BM), dim3(S::THREADS), S::SMEM,
+               stream, A, W + (size_t)n * K, bias ? bias + n : nullptr, C + n, M, part, K, 1, blocks, N);
+  }
   return (int)cudaGetLastError();
 }
 
@@ -238,6 +255,7 @@ int launch_square(int tn, const float* A, const float* W, const float* bias, flo
 VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                        cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
+  if (N > 65535 * 64) return launch_gemm_f32_parts<F32Tile<4, 2, 2, 4, 4, 3, false>>(A, W, bias, C, M, N, K, stream);
   // Rows that 16-byte copies cannot take: odd inner sizes, operands that start between.
   if (K % 4 != 0 || ((uintptr_t)A | (uintptr_t)W) % 16 != 0)
     return launch_gemm_f32<F32Tile<4, 2, 2, 4, 4, 3, false>>(A, W, bias, C, M, N, K, stream);
