@@ -197,6 +197,30 @@ def test_gemm_f32_every_tile_sums_alike(k, N, K, offset):
         assert torch.all(out[M] == 5.0)
 
 
+TILES_F32 = [(tm, tn) for tm in (2, 3, 4, 5, 6, 7, 8, 10) for tn in (4, 8)]
+
+
+@pytest.mark.parametrize("N,K,tiles", [(1152, 896, TILES_F32), (16500, 68, TILES_F32), (200, 301, [(4, 4)]),
+                                       (16390, 70, [(4, 4)])])
+def test_gemm_f32_tiles_asked_for_by_size(k, N, K, tiles):
+    """Every tile that a step can be given, with eight ranges of K and with one, last tiles that are not full:
+    the bits of four rows at a time."""
+    gen = torch.Generator().manual_seed(N)
+    a = torch.randn(87, K, generator=gen).cuda()
+    w, b = torch.randn(N, K, generator=gen).cuda(), torch.randn(N, generator=gen).cuda()
+    want = torch.empty(88, N, device="cuda")
+    for row in range(0, 87, 4):
+        k.gemm_f32(a[row:], w, b, want[row:], min(4, 87 - row))
+    for tile in tiles:
+        for M in (87, 41, 16):
+            out = torch.full((M + 1, N), 5.0, device="cuda")
+            k.gemm_f32(a, w, b, out, M, tile=tile)
+            assert torch.equal(out[:M], want[:M]), (tile, M)
+            assert torch.all(out[M] == 5.0)
+    with pytest.raises(RuntimeError):
+        k.gemm_f32(a, w, b, out, 16, tile=(9, 4))
+
+
 def test_gemm_f32_more_weight_rows_than_a_grid_has_in_y(k):
     """65,535 tiles of 64 weight rows and one more."""
     N = 65535 * 64 + 5

@@ -243,8 +243,8 @@ int launch_gemm_f32_parts(const float* A, const float* W, const float* bias, flo
 using namespace vx;
 
 // Tiles of 2 x 2 warps of 4 x 8 lanes: 8 TM rows x 16 TN weight rows.
-template <int TM, int TN>
-using F32Square = F32Tile<4, 2, 2, TM, TN, 3, true>;
+template <int TM, int TN, bool VEC = true>
+using F32Square = F32Tile<4, 2, 2, TM, TN, 3, VEC>;
 
 template <int TM>
 int launch_square(int tn, const float* A, const float* W, const float* bias, float* C, int M, int N, int K, cudaStream_t s) {
@@ -252,33 +252,39 @@ int launch_square(int tn, const float* A, const float* W, const float* bias, flo
                  : launch_gemm_f32<F32Square<TM, 4>>(A, W, bias, C, M, N, K, s);
 }
 
-VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
+// tile: 16 TM + TN of the tile to take (every one sums alike), 0: the one that takes least.
+VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int tile,
                        cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (N > 65535 * 64) return launch_gemm_f32_parts<F32Tile<4, 2, 2, 4, 4, 3, false>>(A, W, bias, C, M, N, K, stream);
+  if (N > 65535 * 64) return launch_gemm_f32_parts<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
   // Rows that 16-byte copies cannot take: odd inner sizes, operands that start between.
-  if (K % 4 != 0 || ((uintptr_t)A | (uintptr_t)W) % 16 != 0)
-    return launch_gemm_f32<F32Tile<4, 2, 2, 4, 4, 3, false>>(A, W, bias, C, M, N, K, stream);
-  if (M <= 4) return launch_gemm_f32<F32Tile<1, 1, 2, 4, 1, 6, true>>(A, W, bias, C, M, N, K, stream);
-  if (M <= 8) return launch_gemm_f32<F32Tile<1, 1, 2, 8, 1, 6, true>>(A, W, bias, C, M, N, K, stream);
-  // The tile whose launch takes least.  A CTA's time goes with TN (TM + 2.3) (measured with 3 ... 10 rows a
-  // thread and 4 and 8 weight rows, 17,920 x 1,536 at 153 and 260 rows; within 5 %), two share an SM, and one
-  // that has it alone takes three quarters of what two take.  The device holds about 256 CTAs of clusters at
-  // a time (whole clusters in a GPC).
-  const long long ranks = f32_ranks(N, K);
-  int best_tm = 8, best_tn = 8;
-  double best = 1e300;
-  for (int tm : {2, 3, 4, 5, 6, 7, 8, 10})
-    for (int tn : {8, 4}) {
-      const long long ctas = ranks * ((N + 16 * tn - 1) / (16 * tn)) * ((M + 8 * tm - 1) / (8 * tm));
-      double turns = ctas <= 148 ? 1.5 : (double)((ctas + 147) / 148);
-      if (ranks > 1) {
-        const long long rest = ctas % 256;
-        turns = 2.0 * (double)(ctas / 256) + (rest == 0 ? 0.0 : rest <= 148 ? 1.5 : 2.0);
+  if (K % 4 != 0 || ((uintptr_t)A | (uintptr_t)W) % 16 != 0) {
+    if (tile == 0 || tile == 16 * 4 + 4) return launch_gemm_f32<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
+    return (int)cudaErrorInvalidValue;
+  }
+  int best_tm = tile / 16, best_tn = tile % 16;
+  if (tile == 0) {
+    if (M <= 4) return launch_gemm_f32<F32Tile<1, 1, 2, 4, 1, 6, true>>(A, W, bias, C, M, N, K, stream);
+    if (M <= 8) return launch_gemm_f32<F32Tile<1, 1, 2, 8, 1, 6, true>>(A, W, bias, C, M, N, K, stream);
+    // The tile whose launch takes least.  A CTA's time goes with TN (TM + 2.3) (measured with 3 ... 10 rows a
+    // thread and 4 and 8 weight rows, 17,920 x 1,536 at 153 and 260 rows; within 5 %), two share an SM, and one
+    // that has it alone takes three quarters of what two take.  The device holds about 256 CTAs of clusters at
+    // a time (whole clusters in a GPC).
+    const long long ranks = f32_ranks(N, K);
+    double best = 1e300;
+    for (int tm : {2, 3, 4, 5, 6, 7, 8, 10})
+      for (int tn : {8, 4}) {
+        const long long ctas = ranks * ((N + 16 * tn - 1) / (16 * tn)) * ((M + 8 * tm - 1) / (8 * tm));
+        double turns = ctas <= 148 ? 1.5 : (double)((ctas + 147) / 148);
+        if (ranks > 1) {
+          const long long rest = ctas % 256;
+          turns = 2.0 * (double)(ctas / 256) + (rest == 0 ? 0.0 : rest <= 148 ? 1.5 : 2.0);
+        }
+        const double cost = turns * tn * (tm + 2.3 + (tm == 10 ? 0.8 : 0.0));
+        if (cost < best) best = cost, best_tm = tm, best_tn = tn;
       }
-      const double cost = turns * tn * (tm + 2.3 + (tm == 10 ? 0.8 : 0.0));
-      if (cost < best) best = cost, best_tm = tm, best_tn = tn;
-    }
+  }
+  if (best_tn != 4 && best_tn != 8) return (int)cudaErrorInvalidValue;
   switch (best_tm) {
     case 2: return launch_square<2>(best_tn, A, W, bias, C, M, N, K, stream);
     case 3: return launch_square<3>(best_tn, A, W, bias, C, M, N, K, stream);
@@ -287,6 +293,7 @@ VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float*
     case 6: return launch_square<6>(best_tn, A, W, bias, C, M, N, K, stream);
     case 7: return launch_square<7>(best_tn, A, W, bias, C, M, N, K, stream);
     case 8: return launch_square<8>(best_tn, A, W, bias, C, M, N, K, stream);
-    default: return launch_square<10>(best_tn, A, W, bias, C, M, N, K, stream);
+    case 10: return launch_square<10>(best_tn, A, W, bias, C, M, N, K, stream);
+    default: return (int)cudaErrorInvalidValue;
   }
 }

@@ -9,7 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import math
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -51,7 +51,7 @@ def core():
             _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_int, _c_ll, _c_int, _ptr, _ptr,
         ]
         lib.vx_swiglu.argtypes = [_ptr, _ptr, _c_int, _c_int, _c_int, _ptr]
-        lib.vx_gemm_f32.argtypes = [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _ptr]
+        lib.vx_gemm_f32.argtypes = [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr]
         lib.vx_cast_bf16_to_f32.argtypes = [_ptr, _ptr, _c_ll, _ptr]
         lib.vx_sample.argtypes = [
             _ptr, _c_int, _c_int, _c_ll, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_ll, _ptr, _ptr, _ptr, _ptr, _ptr,
@@ -834,8 +834,12 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, num_tokens: int) -> None:
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor,
-             num_rows: int) -> None:
-    """out[:M] = a[:M] @ w.T + bias on the FP32 pipes (true 32-bit, no tensor cores)."""
+             num_rows: int, tile: Optional[Tuple[int, int]] = None) -> None:
+    """out[:M] = a[:M] @ w.T + bias on the FP32 pipes (true 32-bit, no tensor cores).
+
+    ``w`` is a weight: it may be read before the kernel in front of this one on the stream has finished,
+    so that kernel must not write it.  ``tile`` (rows of ``a``, rows of ``w`` a thread) asks for one of the
+    tiles of gemm_f32.cu by its size; all of them give the same bits."""
     _need(a, torch.float32, "a")
     _need(w, torch.float32, "w")
     _need(out, torch.float32, "out")
@@ -846,7 +850,8 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
         _need(bias, torch.float32, "bias")
         if bias.numel() != n:
             raise ValueError("bias length does not match the output width")
-    _check(core().vx_gemm_f32(_p(a), _p(w), _p(bias), _p(out), num_rows, n, k, _stream()), "gemm_f32")
+    code = 0 if tile is None else 16 * tile[0] + tile[1]
+    _check(core().vx_gemm_f32(_p(a), _p(w), _p(bias), _p(out), num_rows, n, k, code, _stream()), "gemm_f32")
 
 
 GEMM_OUT_BF16, GEMM_OUT_F32, GEMM_ADD_F32, GEMM_SWIGLU = 0, 1, 2, 3
