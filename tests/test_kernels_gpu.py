@@ -200,8 +200,8 @@ def test_gemm_f32_every_tile_sums_alike(k, N, K, offset):
 TILES_F32 = [(tm, tn) for tm in (2, 3, 4, 5, 6, 7, 8, 10) for tn in (4, 8)]
 
 
-@pytest.mark.parametrize("N,K,tiles", [(1152, 896, TILES_F32), (16500, 68, TILES_F32), (200, 301, [(4, 4)]),
-                                       (16390, 70, [(4, 4)])])
+@pytest.mark.parametrize("N,K,tiles", [(1152, 896, TILES_F32), (16500, 68, TILES_F32), (200, 301, [(4, 4), (8, 8)]),
+                                       (16390, 70, [(4, 4), (8, 8)])])
 def test_gemm_f32_tiles_asked_for_by_size(k, N, K, tiles):
     """Every tile that a step can be given, with eight ranges of K and with one, last tiles that are not full:
     the bits of four rows at a time."""

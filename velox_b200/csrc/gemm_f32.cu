@@ -259,7 +259,13 @@ VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float*
   if (N > 65535 * 64) return launch_gemm_f32_parts<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
   // Rows that 16-byte copies cannot take: odd inner sizes, operands that start between.
   if (K % 4 != 0 || ((uintptr_t)A | (uintptr_t)W) % 16 != 0) {
-    if (tile == 0 || tile == 16 * 4 + 4) return launch_gemm_f32<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
+    // Tiles of 64 x 128 for many rows, where those of 32 x 64 are 1,024 CTAs and more (us with the small and the large
+    // ones: 2,048 x 1,537 at 260 rows 106 and 92, at 1,024 364 and 276; 9,729 x 898 at 260 rows 217 and 212, at 153
+    // 127 and 142; 200 x 301 at 2,048 rows, 1,024 CTAs, 28.3 and 21.2, at 1,024, 512 CTAs, 15.5 and 17.8).
+    const bool many = M >= 256 && (long long)f32_ranks(N, K) * ((N + 63) / 64) * ((M + 31) / 32) >= 1024;
+    if (tile == 0) tile = many ? 16 * 8 + 8 : 16 * 4 + 4;
+    if (tile == 16 * 4 + 4) return launch_gemm_f32<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
+    if (tile == 16 * 8 + 8) return launch_gemm_f32<F32Square<8, 8, false>>(A, W, bias, C, M, N, K, stream);
     return (int)cudaErrorInvalidValue;
   }
   int best_tm = tile / 16, best_tn = tile % 16;
