@@ -1,11 +1,11 @@
 // float32 GEMM on the FP32 pipes (no tensor cores, no TF32): C[M,N] = A[M,K] * W[N,K]^T + bias.
 //
-// The order of a sum.  K is cut into `ranks` equal ranges of 32-wide blocks, a number that follows from
-// N and K alone (f32_ranks); in a range the products of even k and those of odd k are added up one after
-// the other (the two halves of a packed fma.rn.f32x2), the two sums are added, and the ranges' sums are
-// added in the order of the ranges.  That is the same for every tile shape below, so a row's result does
-// not depend on M or on where the row sits in the batch; and as 2 * ranks shorter chains it is nearer the
-// exact sum than one chain of K.
+// The order of a sum.  K is cut into `ranks` ranges of as many 32-wide blocks each (the last ones may have
+// fewer, or none), a number that follows from N and K alone (f32_ranks); in a range the products of even k
+// and those of odd k are added up one after the other (the two halves of a packed fma.rn.f32x2), the two sums
+// are added, and the ranges' sums are added in the order of the ranges.  That is the same for every tile shape
+// below, so a row's result does not depend on M or on where the row sits in the batch; and as 2 * ranks
+// shorter chains it is nearer the exact sum than one chain of K.
 //
 // How the work is cut.  A CTA makes BM x BN outputs over one range of K; the CTAs of the ranges are a
 // thread-block cluster, which adds up its tiles through distributed shared memory, each CTA a slice of
@@ -14,13 +14,14 @@
 // Pairs along k need no transposed tile and no duplicated operand.
 //   TM 2 ... 10, TN 8 or 4 (9 rows and more): bound by the FP32 pipes and by what two CTAs an SM can hide of
 //   the loads' latency.  TM + TN loads of 16 bytes for 2 TM TN packed FMAs; the weights of the next four k
-//   are read under the products of these (232 -> 211 us for 153 x 17,920 x 1,536).
+//   are read under the products of these (232 -> 211 us for 153 x 17,920 x 1,536 launched alone).
 //   One lane row of 4 or 8 rows (up to eight): bound by the weights' bytes; the rows of A are broadcasts.
 // Weight tiles are asked for before the programmatic-dependency wait.
 //
-// Measured (us; before: one 64 x 64 tile a CTA, 4 x 4 outputs a thread, K in one chain):
-//   153 rows: 17,920 x 1,536 505 -> 211 (40 TFLOP/s), 1,536 x 8,960 667 -> 137, 2,048 x 1,536 119 -> 41;
-//   4 rows: 120 -> 12 (2,048 x 1,536), 700 -> 25 (1,536 x 8,960), 1,070 -> 180 (151,936 x 1,536, 5.2 TB/s).
+// Measured (us back to back in a graph; before: one 64 x 64 tile a CTA, 4 x 4 outputs a thread, K in one chain):
+//   153 rows: 17,920 x 1,536 504 -> 197 (43 TFLOP/s), 1,536 x 8,960 657 -> 128, 2,048 x 1,536 120 -> 31;
+//   4 rows: 702 -> 17.5 (1,536 x 8,960), 1,063 -> 159 (151,936 x 1,536, 5.9 TB/s);
+//   2,048 rows: 17,920 x 1,536 4,390 -> 2,515, 1,152 x 896 207 -> 143.
 // Error against 64 bits (2-norm, normal operands): 7.0e-7 -> 5.0e-7 with one range of 1,536, 1.9e-7 with
 // eight; 1.7e-6 -> 4.3e-7 with 8,960 in eight.
 #include "common.cuh"
@@ -197,8 +198,10 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, const 
   cluster_meet();  // nobody leaves while a peer reads its tile
 }
 
-// Ranges of K: enough CTAs of 64 weight rows for two on every SM of a 148-SM device, at least two
-// 32-wide blocks a range.  From N and K alone: the order of a sum must not depend on anything else.
+// Ranges of K: enough CTAs of 64 weight rows for two on every SM of a 148-SM device, as long as that is two
+// 32-wide blocks a range on average.  A range has as many whole blocks as the mean rounded up, so less is left for
+// the last ones (28 blocks in eight ranges: seven of four and an empty one).  From N and K alone: the order of
+// a sum must not depend on anything else.
 inline int f32_ranks(int N, int K) {
   const int tiles = (N + 63) / 64, blocks = (K + F32_BK - 1) / F32_BK;
   int ranks = 1;
@@ -275,7 +278,8 @@ VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float*
     // The tile whose launch takes least.  A CTA's time goes with TN (TM + 2.3) (measured with 3 ... 10 rows a
     // thread and 4 and 8 weight rows, 17,920 x 1,536 at 153 and 260 rows; within 5 %), two share an SM, and one
     // that has it alone takes three quarters of what two take.  The device holds about 256 CTAs of clusters at
-    // a time (whole clusters in a GPC).
+    // a time (whole clusters in a GPC).  Over the projections of the 0.5B and 1.5B sizes at 12 ... 2,048 rows the
+    // choice takes as long as the best of the tiles within 10 % in 60 of 70 cases, 26 % longer at most (1,152 x 896 at 100 rows).
     const long long ranks = f32_ranks(N, K);
     double best = 1e300;
     for (int tm : {2, 3, 4, 5, 6, 7, 8, 10})
