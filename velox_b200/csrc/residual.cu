@@ -299,8 +299,8 @@ __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v
 
 // FEW rows (bfloat16 steps of a few tokens): a thread has one chunk, and the depth mix asks for eight earlier results at a
 // time, ahead of the reductions that do not need them.  One after the other they were 12.7 us a launch of eight rows on average
-over 28 layers, bound by the latency of a chain of loads; a step of 8 tokens takes 2,003 us where it took 2,153 (with
-the few-token products).  A portion of 700 tokens is slower this way (4.23 ms against 4.13), hence a form for few rows.
+// over 28 layers, bound by the latency of a chain of loads; a step of 8 tokens takes 2,003 us where it took 2,153 (with
+// the few-token products).  A portion of 700 tokens is slower this way (4.23 ms against 4.13), hence a form for few rows.
 template <typename T, int CHUNKS, bool FEW>
 __global__ void gated_norm_add_vec_kernel(const float* resid_in, float* resid_out, const T* __restrict__ delta,
                                           long long delta_ld, const T* __restrict__ gate, long long gate_ld,
