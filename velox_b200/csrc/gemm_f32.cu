@@ -259,7 +259,7 @@ int launch_square(int tn, const float* A, const float* W, const float* bias, flo
 }
 
 VX_API long long vx_gemm_f32_scratch(const float* A, const float* W, int M, int N, int K, int tile) {
-  return tile == 0 && M > 0 && N > 0 && gemm_f32_tc_takes(A, W, M, N, K) ? gemm_f32_tc_scratch(M, K) : 0;
+  return tile == 0 && M > 0 && N > 0 && gemm_f32_tc_takes(A, W, N, K) ? gemm_f32_tc_scratch(M, K) : 0;
 }
 
 // tile: 16 TM + TN of the tile to take (every one sums alike), 0: the one that takes least.
@@ -267,7 +267,7 @@ VX_API long long vx_gemm_f32_scratch(const float* A, const float* W, int M, int 
 VX_API int vx_gemm_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, int tile, void* scratch,
                        int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
-  if (tile == 0 && gemm_f32_tc_takes(A, W, M, N, K)) return gemm_f32_tc(A, W, bias, C, M, N, K, scratch, status, stream);
+  if (tile == 0 && gemm_f32_tc_takes(A, W, N, K)) return gemm_f32_tc(A, W, bias, C, M, N, K, scratch, status, stream);
   if (N > 65535 * 64) return launch_gemm_f32_parts<F32Square<4, 4, false>>(A, W, bias, C, M, N, K, stream);
   // Rows that 16-byte copies cannot take: odd inner sizes, operands that start between.
   if (K % 4 != 0 || ((uintptr_t)A | (uintptr_t)W) % 16 != 0) {

@@ -42,6 +42,7 @@ constexpr int FT_A_COLS = FT_TERMS * FT_BK / 2;  // columns of tensor memory of 
 constexpr uint32_t FT_W_BYTES = UMMA_M * FT_BK * 4;
 constexpr int FT_MAX_RANKS = 8;
 constexpr int FT_PITCH = UMMA_M + 4;     // of a token's row in the exchange
+constexpr int FT_LAUNCH_ROWS = 8000;     // rows of A at a time: bounds the scratch, and the grid of clusters (at most 56 tiles of W)
 
 template <int BN_>
 struct F32Tensor {
@@ -557,28 +558,37 @@ static int launch_gemm_f32_tc(const CUtensorMap& map, F32TensorArgs g, __nv_bflo
 // row, 35.5 -> 22.1 at eight, 196 -> 48 at 153; 1,536 x 8,960 16.9 -> 16.9, 23.1 -> 17.4, 128 -> 37; 151,936 x 1,536 151 -> 158, 181 -> 159,
 // 442 -> 233 at 40.  Smaller ones have too few CTAs of 128 rows for a few rows of A, and a row must have the same bits in every
 // step: 9,728 x 896 8.7 -> 12.9 at one row (88 -> 29 at 153), 2,048 x 1,536 4.9 -> 7.4 (31 -> 17).
-bool gemm_f32_tc_takes(const float* A, const float* W, int M, int N, int K) {
-  // (A grid has 65,535 items in y.)
-  return K >= 512 && (long long)N * K >= 12 << 20 && K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0 &&
-         ((long long)N + UMMA_M - 1) / UMMA_M * ((M + 159) / 160) <= 65535 && M <= (1 << 24);
+bool gemm_f32_tc_takes(const float* A, const float* W, int N, int K) {
+  return K >= 512 && (long long)N * K >= 12 << 20 && K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
 }
 
-long long gemm_f32_tc_scratch(int M, int K) { return M <= 16 ? 0 : (long long)FT_TERMS * M * f32_tc_pitch(K) * 2; }
+long long gemm_f32_tc_scratch(int M, int K) {
+  return M <= 16 ? 0 : (long long)FT_TERMS * (M < FT_LAUNCH_ROWS ? M : FT_LAUNCH_ROWS) * f32_tc_pitch(K) * 2;
+}
 
-int gemm_f32_tc(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, void* scratch, int* status,
-                cudaStream_t stream) {
-  CUtensorMap map;
-  if (!ft_tensor_map(&map, W, N, K)) return (int)cudaErrorInvalidValue;
-  const F32TensorArgs g = {A, W, bias, C, status, M, N, K, 1, 0, 1, 0};
-  __nv_bfloat16* const terms = (__nv_bfloat16*)scratch;
+// One launch: at most FT_LAUNCH_ROWS rows.
+static int gemm_f32_tc_rows(const CUtensorMap& map, const F32TensorArgs& g, __nv_bfloat16* terms, cudaStream_t stream) {
   // Rows in as few tiles as take up to 160 each, and those as narrow as they can be.
-  const int tiles = (M + 159) / 160, rows = (M + tiles - 1) / tiles;
+  const int M = g.M, tiles = (M + 159) / 160, rows = (M + tiles - 1) / tiles;
   if (M <= 16) return launch_gemm_f32_tc<16>(map, g, terms, stream);
   if (rows <= 32) return launch_gemm_f32_tc<32>(map, g, terms, stream);
   if (rows <= 64) return launch_gemm_f32_tc<64>(map, g, terms, stream);
   if (rows <= 96) return launch_gemm_f32_tc<96>(map, g, terms, stream);
   if (rows <= 128) return launch_gemm_f32_tc<128>(map, g, terms, stream);
   return launch_gemm_f32_tc<160>(map, g, terms, stream);
+}
+
+int gemm_f32_tc(const float* A, const float* W, const float* bias, float* C, int M, int N, int K, void* scratch, int* status,
+                cudaStream_t stream) {
+  CUtensorMap map;
+  if (!ft_tensor_map(&map, W, N, K)) return (int)cudaErrorInvalidValue;
+  // (A launch's first kernel waits for the launch before it, whose split rows lie in the same scratch.)
+  for (int m = 0;; m += FT_LAUNCH_ROWS) {
+    const bool last = M - m <= FT_LAUNCH_ROWS;
+    const F32TensorArgs g = {A + (size_t)m * K, W, bias, C + (size_t)m * N, status, last ? M - m : FT_LAUNCH_ROWS, N, K, 1, 0, 1, 0};
+    const int code = gemm_f32_tc_rows(map, g, (__nv_bfloat16*)scratch, stream);
+    if (code != 0 || last) return code;
+  }
 }
 
 }  // namespace vx

@@ -2,7 +2,8 @@
 
 float32: this package's own GEMM, always (no TF32, no library): small matrices on the FP32 pipes, large ones on the
 tensor cores as products of three-term bfloat16 splits with float32 sums, nearer the exact sums than a chain of FMAs.
-Which of the two follows from the matrix alone, and every output element is summed in a fixed order.
+Which of the two follows from the matrix alone (rows that do not begin at multiples of 16 bytes stay on the
+FP32 pipes), and every output element is summed in a fixed order.
 
 bfloat16: the tcgen05/TMA kernel of ``csrc/gemm_bf16.cu`` when the step has few tokens (decode
 and short portions: the weight fills the 128-row side of the tensor-core tile and is streamed
