@@ -4,10 +4,11 @@
 // The numbers.  A float32 is the sum of three bfloat16 numbers, the value rounded, what that left rounded, and
 // what both left (8 + 8 + 8 bits and their signs: nothing is lost unless the third is below 2^-133).  Of the nine
 // products of two such sums the six of order 2^-16 and above are taken, each exact in the tensor core's
-// float32 accumulator; what is left out is below 2^-25 of the product.  The accumulator does not
+// float32 accumulator; what is left out is below 2^-24 of the product (two of up to 2^-25).  The accumulator does not
 // round to nearest, so sums do not grow in it: a chunk of 32 of the inner dimension is made there, smallest
 // products first, and added to the running sum in registers, which is an ordinary float32 addition.
-// A sum that is not finite is made again by FMAs from the operands (infinities have no such split).
+// A sum that is not finite, or below 2^-96, is made again by FMAs from the operands (infinities have no such split, and the
+// third terms of tiny operands are lost).
 //
 // Error against 64 bits (2-norm, normal operands): 9.0e-8 with K 1,536 (an FMA chain in one range 3.0e-7), 1.2e-7 with 8,960 in eight
 // ranges (3.8e-7).
@@ -170,13 +171,57 @@ __device__ __forceinline__ void ft_add2(float& s0, float& s1, uint32_t p0, uint3
       : "r"(p0), "r"(p1));
 }
 
-__device__ __forceinline__ bool ft_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+// Sums that the split makes.  Not among them: those with infinities or NaN, and those so small that their operands' third
+// terms are below bfloat16's smallest number (operands below 2^-109 beside others of up to 2^13 over sqrt(K)).
+__device__ __forceinline__ bool ft_regular(float v) {
+  const float size = fabsf(v);
+  return size <= 3.402823466e38f && (size >= 0x1p-96f || size == 0.f);
+}
 
-// One element from the operands, for sums that the split cannot make.
-__device__ __noinline__ float ft_by_fma(const float* a, const float* w, int K, float add) {
+// Whether a row has a NaN (the whole warp; K is a multiple of four, the row starts at 16 bytes).
+__device__ __noinline__ bool ft_has_nan(const float* row, int K) {
+  bool found = false;
+#pragma unroll 4
+  for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(row + k));
+    found = found || v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w;
+  }
+  return __any_sync(0xffffffffu, found);
+}
+
+// A row times a row by FMAs, an order that follows from K alone (the whole warp).
+__device__ __noinline__ float ft_dot(const float* a, const float* w, int K) {
   float sum = 0.f;
-  for (int k = 0; k < K; ++k) sum = fmaf(a[k], w[k], sum);
-  return sum + add;
+#pragma unroll 4
+  for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
+    const float4 x = __ldcg(reinterpret_cast<const float4*>(a + k)), y = __ldcg(reinterpret_cast<const float4*>(w + k));
+    sum = fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, sum))));
+  }
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, step);
+  return sum;
+}
+
+// Makes those of 32 elements (row `a` with weight rows `first` on, one a lane) again that `bad` names; the whole warp, every
+// lane brings and gets its element.  A NaN in a row or a weight row is an answer without the products; `known` and
+// `nans` remember what was found in the weight rows.  (One thread an element, one after the other, took 17.4 ms for 153 rows of
+// NaN by 17,920 x 1,536, the FP32 pipes 0.19.)
+__device__ __noinline__ float ft_again(const float* a, const float* W, int first, int K, uint32_t bad, uint32_t* known, uint32_t* nans,
+                                       float element) {
+  const int lane = threadIdx.x & 31;
+  const float nan = __int_as_float(0x7fc00000);
+  if (ft_has_nan(a, K)) return (bad >> lane & 1u) != 0 ? nan : element;
+  for (uint32_t left = bad; left != 0; left &= left - 1) {
+    const int at = __ffs((int)left) - 1;
+    const float* const w = W + (size_t)(first + at) * K;
+    if ((*known >> at & 1u) == 0) {
+      *known |= 1u << at;
+      if (ft_has_nan(w, K)) *nans |= 1u << at;
+    }
+    const float sum = (*nans >> at & 1u) != 0 ? nan : ft_dot(a, w, K);
+    if (lane == at) element = sum;
+  }
+  return element;
 }
 
 template <typename S>
@@ -429,22 +474,29 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         continue;
       }
       const int n = n0 + row;
-      if (n >= g.N) continue;
-      const float add = g.bias != nullptr ? g.bias[n] : 0.f;
-      bool finite = true;
+      const bool there = n < g.N;
+      const float add = g.bias != nullptr && there ? g.bias[n] : 0.f;
+      // (What is to be made again is marked by a NaN.)
+      bool regular = true;
 #pragma unroll
       for (int j = 0; j < S::PART; ++j) {
         const int m = m0 + half * S::PART + j;
-        if (m >= g.M) continue;
-        finite = finite && ft_finite(sum[j]);
-        g.C[(size_t)m * g.N + n] = sum[j] + add;
+        if (m >= g.M || !there) continue;
+        const bool good = ft_regular(sum[j]);
+        regular = regular && good;
+        g.C[(size_t)m * g.N + n] = good ? sum[j] + add : __int_as_float(0x7fc00000);
       }
-      if (!finite && ok)
-        for (int j = 0; j < S::PART; ++j) {
+      if (ok && __any_sync(0xffffffffu, !regular)) {
+        uint32_t known = 0, nans = 0;
+        for (int j = 0; j < S::PART && m0 + half * S::PART + j < g.M; ++j) {
           const int m = m0 + half * S::PART + j;
-          if (m < g.M && !ft_finite(g.C[(size_t)m * g.N + n]))
-            g.C[(size_t)m * g.N + n] = ft_by_fma(g.A + (size_t)m * g.K, g.W + (size_t)n * g.K, g.K, add);
+          float* const at = g.C + (size_t)m * g.N + n;
+          const uint32_t bad = __ballot_sync(0xffffffffu, there && isnan(*at));
+          if (bad == 0) continue;
+          const float again = ft_again(g.A + (size_t)m * g.K, g.W, n0 + quarter * 32, g.K, bad, &known, &nans, 0.f);
+          if ((bad >> lane & 1u) != 0) *at = again + add;
         }
+      }
     }
   }
   if (g.ranks > 1) {
@@ -458,9 +510,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
     for (int r = 0; r < FT_MAX_RANKS; ++r) peers[r] = r < g.ranks ? peer_address(smem_p, r) : 0u;
     for (int e = rank * S::THREADS + threadIdx.x; e < BN * UMMA_M; e += g.ranks * S::THREADS) {
+      // (A warp has 32 weight rows of one m.)
       const int m = m0 + e / UMMA_M, n = n0 + e % UMMA_M;
       if (m >= g.M) break;
-      if (n >= g.N) continue;
       float part[FT_MAX_RANKS];
 #pragma unroll
       for (int r = 0; r < FT_MAX_RANKS; ++r)
@@ -473,8 +525,12 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
       for (int r = 1; r < FT_MAX_RANKS; ++r)
         if (r < g.ranks) sum += part[r];
-      const float add = g.bias != nullptr ? g.bias[n] : 0.f;
-      g.C[(size_t)m * g.N + n] = ft_finite(sum) ? sum + add : ft_by_fma(g.A + (size_t)m * g.K, g.W + (size_t)n * g.K, g.K, add);
+      const uint32_t bad = __ballot_sync(0xffffffffu, n < g.N && !ft_regular(sum));
+      if (bad != 0) {
+        uint32_t known = 0, nans = 0;
+        sum = ft_again(g.A + (size_t)m * g.K, g.W, n - lane, g.K, bad, &known, &nans, sum);
+      }
+      if (n < g.N) g.C[(size_t)m * g.N + n] = sum + (g.bias != nullptr ? g.bias[n] : 0.f);
     }
     cluster_meet();  // nobody leaves while a peer reads its tile
   }
