@@ -206,50 +206,25 @@ __global__ void delta_rule_scan_kernel(const float* __restrict__ packed, long lo
     const float* buf = dr_smem + (size_t)stage * TT * token_floats;
     const float* tok = buf + p * DR_KP;
     int row_now = t_first + index * TT;
-    // A token's vectors, this thread's rows of them.  With four rows a thread the next token's are read before this one's
-    // shuffles, so that the chain from token to token has no shared-memory read on it.
-    constexpr int K_AT = FORM == DR_GENERAL ? 3 * KD : FORM == DR_CHANNEL ? KD : 0;
-    constexpr int Q = DR_KP / 4;
-    constexpr bool AHEAD = Q == 1;
-    struct Token {
-      float4 w[Q], a[Q], u[Q], k[Q], r[Q];
-      float2 gb;  // g (DR_HEAD), beta
-      float v;
-    };
-    const auto read = [&](const float* at, Token& t) {
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        t.k[q] = reinterpret_cast<const float4*>(at + K_AT)[q];
-        t.r[q] = reinterpret_cast<const float4*>(at + K_AT + KD)[q];
-        if constexpr (FORM != DR_HEAD) t.w[q] = reinterpret_cast<const float4*>(at)[q];
-        if constexpr (FORM == DR_GENERAL) {
-          t.a[q] = reinterpret_cast<const float4*>(at + KD)[q];
-          t.u[q] = reinterpret_cast<const float4*>(at + 2 * KD)[q];
-        }
-      }
-      if constexpr (FORM != DR_GENERAL) t.gb = *reinterpret_cast<const float2*>(at + vec - p * DR_KP - 2);
-      t.v = value_col ? at[vec - p * DR_KP + col] : 0.f;
-    };
-    Token now, after;
-    if (AHEAD) read(tok, now);
 #pragma unroll 2
     for (int i = 0; i < tt; ++i, tok += token_floats, ++row_now) {
-      if (AHEAD) {
-        if (i + 1 < tt) read(tok + token_floats, after);
-      } else {
-        read(tok, now);
-      }
+      constexpr int K_AT = FORM == DR_GENERAL ? 3 * KD : FORM == DR_CHANNEL ? KD : 0;
+      const float4* w4 = reinterpret_cast<const float4*>(tok);
+      const float4* a4 = reinterpret_cast<const float4*>(tok + KD);
+      const float4* u4 = reinterpret_cast<const float4*>(tok + 2 * KD);
+      const float4* k4 = reinterpret_cast<const float4*>(tok + K_AT);
+      const float4* r4 = reinterpret_cast<const float4*>(tok + K_AT + KD);
       float us0 = 0.f, us1 = 0.f, us2 = 0.f, us3 = 0.f;
       float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
+      for (int q = 0; q < DR_KP / 4; ++q) {
         float4 u;
         if constexpr (FORM == DR_GENERAL) {
-          u = now.u[q];
+          u = u4[q];
         } else if constexpr (FORM == DR_HEAD) {
-          u = now.k[q];  // the decay multiplies the finished sum
+          u = k4[q];  // the decay multiplies the finished sum
         } else {
-          const float4 w = now.w[q], k = now.k[q];
+          const float4 w = w4[q], k = k4[q];
           u = make_float4(w.x * k.x, w.y * k.y, w.z * k.z, w.w * k.w);
         }
         us0 = fmaf(u.x, S[4 * q], us0);
@@ -271,24 +246,24 @@ __global__ void delta_rule_scan_kernel(const float* __restrict__ packed, long lo
         }
       }
       if (pending && mode != 1 && live && p == 0) out[(size_t)pending_row * out_stride + (size_t)h * Dv + col] = o;
-      const float vj = now.v;
+      const float vj = value_col ? tok[vec - p * DR_KP + col] : 0.f;
       if constexpr (FORM == DR_GENERAL) {
 #pragma unroll
         for (int q = 0; q < DR_KP / 4; ++q) {
-          const float4 w = now.w[q], a = now.a[q], k = now.k[q];
+          const float4 w = w4[q], a = a4[q], k = k4[q];
           S[4 * q] = fmaf(w.x, S[4 * q], fmaf(-a.x, us, k.x * vj));
           S[4 * q + 1] = fmaf(w.y, S[4 * q + 1], fmaf(-a.y, us, k.y * vj));
           S[4 * q + 2] = fmaf(w.z, S[4 * q + 2], fmaf(-a.z, us, k.z * vj));
           S[4 * q + 3] = fmaf(w.w, S[4 * q + 3], fmaf(-a.w, us, k.w * vj));
         }
       } else {
-        const float2 gb = now.gb;
+        const float2 gb = *reinterpret_cast<const float2*>(tok + vec - p * DR_KP - 2);  // g (DR_HEAD), beta
         const float change = FORM == DR_HEAD ? gb.y * fmaf(-gb.x, us, vj) : gb.y * (vj - us);
 #pragma unroll
         for (int q = 0; q < DR_KP / 4; ++q) {
-          const float4 k = now.k[q];
+          const float4 k = k4[q];
           float4 w = make_float4(gb.x, gb.x, gb.x, gb.x);
-          if constexpr (FORM == DR_CHANNEL) w = now.w[q];
+          if constexpr (FORM == DR_CHANNEL) w = w4[q];
           S[4 * q] = fmaf(w.x, S[4 * q], k.x * change);
           S[4 * q + 1] = fmaf(w.y, S[4 * q + 1], k.y * change);
           S[4 * q + 2] = fmaf(w.z, S[4 * q + 2], k.z * change);
@@ -297,7 +272,7 @@ __global__ void delta_rule_scan_kernel(const float* __restrict__ packed, long lo
       }
 #pragma unroll
       for (int q = 0; q < DR_KP / 4; ++q) {
-        const float4 r = now.r[q];
+        const float4 r = r4[q];
         r_prev[4 * q] = r.x;
         r_prev[4 * q + 1] = r.y;
         r_prev[4 * q + 2] = r.z;
@@ -305,7 +280,6 @@ __global__ void delta_rule_scan_kernel(const float* __restrict__ packed, long lo
       }
       pending = true;
       pending_row = row_now;
-      if (AHEAD) now = after;
     }
     __syncthreads();  // every thread is done with this stage before it is filled again
     if (threadIdx.x == 0 && index + 2 < num_tiles) issue(index + 2);
