@@ -110,3 +110,15 @@ def test_refuses_what_its_copies_cannot_take(k, status):
     w = torch.zeros(256, 60, dtype=torch.bfloat16, device="cuda")
     out = torch.zeros(300, 256, device="cuda")
     assert not k.gemm_bf16_wide(x, w, None, out, k.GEMM_ADD_F32, 300, status)
+
+
+def test_sums_beyond_768_tokens_repeat(k, status):
+    """One chunk of the inner size: an element has one addition, whatever ran before."""
+    _, x, w = _operands(1030, 1536, 8960)
+    first = None
+    for _ in range(6):
+        stream = torch.ones(1030, 1536, device="cuda")
+        assert k.gemm_bf16_wide(x, w, None, stream, k.GEMM_ADD_F32, 1030, status)
+        first = stream if first is None else first
+        assert torch.equal(stream, first)
+    assert int(status[0]) == 0

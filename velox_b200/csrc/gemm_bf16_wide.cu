@@ -15,9 +15,9 @@
 // BN is a multiple of 16 up to 256, chosen so that the tiles come out even over the pairs (choose_tile).
 //
 // Epilogues:
-//   2  out f32 [T, ldy] += acc + bias: a projection straight into the residual stream.  Where the tiles do not come out
-//      even over the pairs K is cut into chunks, each a tile's item of its own that adds its share (the order of those
-//      additions is not fixed; with one chunk an element has one addition)
+//   2  out f32 [T, ldy] += acc + bias: a projection straight into the residual stream.  Up to 768 tokens, where the tiles do
+//      not come out even over the pairs, K is cut into chunks, each a tile's item of its own that adds its share (the order of
+//      those additions is not fixed; with one chunk an element has one addition)
 //   3  out bf16 [T, ldy] = silu(gate) * up of W = N gate rows, then N up rows: the tensor map deals the rows in turn, so
 //      that neighbouring lanes hold gate and up of a feature and hand each other one of two tokens
 //   6  mode 3 with the options of the gated activation (GluArgs of gemm_bf16.cu: biases [2 N], clamps, the sigmoid's slope
@@ -432,6 +432,10 @@ static void choose_tile(int T, int weight_tiles, int blocks, int pairs, int most
     }
 }
 
+// Sums of this many tokens at most may cut K: 1,024 tokens of the 14B output projection took 64 us in one chunk and 73 in several,
+// 2,048 tokens 89 and 106, of the down projections 214 and 214, 198 and 203 (7B), 46 and 46 (1.5B).
+constexpr int GW_CHUNKED_TOKENS = 768;
+
 template <int MODE>
 static int launch_wide(const CUtensorMap& mw, const CUtensorMap& mx, const WideArgs& g, int pairs, cudaStream_t stream) {
   static const cudaError_t ready =
@@ -454,7 +458,7 @@ static int gemm_bf16_wide(const void* x, int x_rows, const void* w, int mode, Wi
   const int weight_tiles = (rows + 2 * UMMA_M - 1) / (2 * UMMA_M), pairs = gw_pairs();
   const int blocks = (K + GW_BK - 1) / GW_BK;
   if (chunks < 0 || (chunks > 1 && mode != 2)) return -1;
-  choose_tile(T, weight_tiles, blocks, pairs, chunks != 0 ? 1 : mode == 2 ? 8 : 1, g.bn, g.chunks);
+  choose_tile(T, weight_tiles, blocks, pairs, chunks == 0 && mode == 2 && T <= GW_CHUNKED_TOKENS ? 8 : 1, g.bn, g.chunks);
   if (tokens != 0) g.bn = tokens;
   if (chunks != 0) g.chunks = chunks < blocks ? chunks : blocks;
   g.blocks_per_chunk = (blocks + g.chunks - 1) / g.chunks;

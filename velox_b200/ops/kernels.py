@@ -922,7 +922,7 @@ def gemm_bf16_wide(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
                    num_rows: int, status: torch.Tensor, tokens: int = 0, chunks: int = 0) -> bool:
     """``gemm_bf16`` for steps of many rows, on pairs of SMs (gemm_bf16_wide.cu): modes
     ``GEMM_ADD_F32`` and ``GEMM_SWIGLU``.  ``tokens`` of a tile and ``chunks`` of the inner size (``GEMM_ADD_F32`` only;
-    with more than one the order of an element's additions is not fixed): 0 for what takes least.  False (nothing
+    with more than one the order of an element's additions is not fixed): 0 for what takes least (one chunk beyond 768 rows).  False (nothing
     launched) for sizes that the kernel refuses."""
     _need(x, torch.bfloat16, "x")
     _need(w, torch.bfloat16, "w")
