@@ -112,6 +112,20 @@ def test_refuses_what_its_copies_cannot_take(k, status):
     assert not k.gemm_bf16_wide(x, w, None, out, k.GEMM_ADD_F32, 300, status)
 
 
+# (tokens, N, K, mode): both sides of the lines as they were measured, and of what they are drawn between.
+@pytest.mark.parametrize("T,N,K,mode,chunked,pays", [
+    (300, 1536, 8960, 2, True, True), (300, 1536, 8960, 2, False, False), (768, 1536, 8960, 2, True, True),
+    (769, 1536, 8960, 2, True, False), (300, 1536, 1536, 2, True, True), (300, 1536, 1536, 2, False, True),
+    (768, 2048, 2048, 2, True, True), (769, 2048, 2048, 2, True, False), (536, 3584, 3584, 2, True, False),
+    (2048, 3584, 3584, 2, True, True), (2048, 3584, 3584, 2, False, True), (1400, 3584, 18944, 2, True, False),
+    (2048, 8960, 1536, 3, True, True), (300, 8960, 1536, 3, True, True), (1755, 4864, 896, 3, True, True),
+    (1756, 4864, 896, 3, True, False), (536, 18944, 3584, 3, True, True), (300, 18944, 3584, 3, True, False),
+    (2048, 18944, 3584, 6, True, True), (700, 8960, 1536, 6, True, False), (2048, 20736, 5120, 5, True, True),
+    (700, 12544, 2048, 5, True, False)])
+def test_which_products_pay(k, T, N, K, mode, chunked, pays):
+    assert k.gemm_bf16_wide_pays(mode, T, N, K, chunked) is pays
+
+
 def test_sums_beyond_768_tokens_repeat(k, status):
     """One chunk of the inner size: an element has one addition, whatever ran before."""
     _, x, w = _operands(1030, 1536, 8960)
@@ -121,4 +135,33 @@ def test_sums_beyond_768_tokens_repeat(k, status):
         assert k.gemm_bf16_wide(x, w, None, stream, k.GEMM_ADD_F32, 1030, status)
         first = stream if first is None else first
         assert torch.equal(stream, first)
+    assert int(status[0]) == 0
+
+
+# One product after the other on pairs of SMs and in the library, in all four ways.
+@pytest.mark.parametrize("T,E,I,gate,down", [(300, 896, 4864, True, True), (1000, 1536, 8960, True, False),
+                                             (300, 3584, 9000, False, True), (1800, 896, 4864, False, False)])
+def test_feed_forward_on_both_sides_of_the_lines(k, status, T, E, I, gate, down):
+    from types import SimpleNamespace
+
+    from velox_b200.engine.runner import Workspace
+    from velox_b200.parts.mlp import SwiGLU
+
+    assert k.gemm_bf16_wide_pays(k.GEMM_SWIGLU, T, I, E, True) is gate and k.gemm_bf16_wide_pays(k.GEMM_ADD_F32, T, E, I, True) is down
+    gen, x, w = _operands(T, 2 * I, E)
+    w_down = (torch.randn(E, I, generator=gen) / math.sqrt(I)).to(torch.bfloat16).cuda()
+    part = SwiGLU({"hidden_size": E, "intermediate_size": I}, {"gate_up.weight": w, "down.weight": w_down}, torch.bfloat16,
+                  torch.device("cuda"))
+    start = torch.randn(T + 3, E, generator=gen).cuda()
+    stream = start.clone()
+    ctx = SimpleNamespace(num_tokens=T, workspace=Workspace(T + 3, 8, torch.device("cuda")), residual=stream, status=status)
+    out = part.forward(x, ctx)
+    assert (out is None) is down
+    both = x[:T].double() @ w.double().T
+    want = (torch.nn.functional.silu(both[:, :I]) * both[:, I:]) @ w_down.double().T
+    # The activation and, from the library, the product are rounded to bfloat16 (2^-9 of them); sums of I like errors.
+    bound = 2.0 ** -7 * want.abs().max().item()
+    got = stream - start if down else out
+    assert (got[:T].double() - want).abs().max().item() <= bound
+    assert torch.equal(stream[T:], start[T:]) and (down or torch.equal(stream, start))
     assert int(status[0]) == 0

@@ -26,7 +26,7 @@
 //
 // Every wait is bounded; a thread that gives up sets a status bit, and the CTAs still meet at the end and free
 // their tensor memory.
-// A projection with nothing of this behind it stays with the library: the plain form took 15 us against 12 (2,048 tokens,
+// Which products come here is said by gw_pays.  A projection with nothing of this behind it stays with the library: the plain form took 15 us against 12 (2,048 tokens,
 // 2048 x 1536), 20 against 15 (536, 4608 x 3584), 25 against 15 (2,048, 896 x 4864), equal at 7168 x 5120; with rotation
 // and cache write in the epilogue 29, 40 and 134 us against the library's 12, 15 and 104 and the 4 - 14 us of a kernel behind
 // it: a row of the accumulator is a feature, and the cache's and the output's lines are written two bytes a lane and token.
@@ -411,12 +411,12 @@ static int gw_pairs() {
   return pairs;
 }
 
-// Tokens of a tile and chunks of K: rounds of items over the pairs times an item's time, in cycles.  A block of K takes what its
-// operands (16 KB + 64 bn bytes a CTA) take into shared memory, 43 bytes a cycle and SM as measured, which is longer than its
-// products at every bn.  Sums into the stream are bound by the L2's additions where items are short (49 cycles a token and pair
-// with all pairs at it); the last item's epilogue is not covered by another's products.  Within a few per cent of the best
-// of 5 tiles x 6 numbers of chunks for the projections of the 0.5B to 14B sizes at 260 to 2,048 tokens.
-static void choose_tile(int T, int weight_tiles, int blocks, int pairs, int most_chunks, int& bn_out, int& chunks_out) {
+// Tokens of a tile and chunks of K: rounds of items over the pairs times an item's time, in cycles, which is returned.  A block of
+// K takes what its operands (16 KB + 64 bn bytes a CTA) take into shared memory, 43 bytes a cycle and SM as measured, which is longer
+// than its products at every bn.  Sums into the stream by chunks are bound by the L2's additions where items are short (49 cycles a
+// token and pair with all pairs at it); the last item's epilogue is not covered by another's products.  Within a few per cent of
+// the best of 5 tiles x 6 numbers of chunks for the projections of the 0.5B to 14B sizes at 260 to 2,048 tokens.
+static double choose_tile(int T, int weight_tiles, int blocks, int pairs, int most_chunks, int& bn_out, int& chunks_out) {
   double least = 1e300;
   const bool sums = most_chunks > 1;
   for (int chunks = 1; chunks <= most_chunks; ++chunks)
@@ -430,11 +430,42 @@ static void choose_tile(int T, int weight_tiles, int blocks, int pairs, int most
       if (chunks > 1) cost *= 1.10;  // (one chunk has one order of additions, and the model flatters many)
       if (cost < least) least = cost, bn_out = bn, chunks_out = chunks;
     }
+  return least;
 }
 
 // Sums of this many tokens at most may cut K: 1,024 tokens of the 14B output projection took 64 us in one chunk and 73 in several,
 // 2,048 tokens 89 and 106, of the down projections 214 and 214, 198 and 203 (7B), 46 and 46 (1.5B).
 constexpr int GW_CHUNKED_TOKENS = 768;
+
+// Whether a product is better off here than as a library product with the kernel that follows it.  Measured (library -> here, us):
+// both in graphs at 26 numbers of tokens between 257 and 6,000 of the 0.5B to 14B sizes, and whole steps, replayed and queued
+// launch by launch.  Queued so, steps of the narrower models are bound by the host to about 1.5 Mi numbers of a stream (0.5B 1,755
+// tokens, 1.5B 1,024, 3B 768), and a library product with its follower costs the host some 10 us more: there a few us of the
+// device's time are given for it.
+//   Sums, K the longer side (down), cut into chunks: 257 tokens 0.5B 11 -> 10, 1.5B 18 -> 14, 3B 21 -> 19, 7B 55 -> 44, 14B 63 -> 63; 536 tokens 12 ->
+//     13, 21 -> 18, 34 -> 25, 63 -> 62, 73 -> 70.
+//   Other sums (in one chunk beyond 768 tokens) pay where the tiles come out even, that is where the cost above leaves the tensor cores 49 % of
+//     their time: 2,048 tokens 7B 54 -> 47 (output), 204 -> 198 (down), 14B 97 -> 89, 225 -> 214; from 0.92 to 1.13 times as fast; at 1,400
+//     tokens 7B 35 -> 39, 138 -> 172 with 43 %.  Output projections come here where the host is the bound: 300 tokens
+//     0.5B 5.8 -> 7.9, 1.5B 7.3 -> 8.6, 3B 8.9 -> 10.0; a step of them replayed takes up to 1 % more, queued 2,582 us where it took 2,830, 2,946
+//     where 3,216, 3,695 where 4,053.
+//   SwiGLU pays with 47 % (2,048 tokens 1.5B 90 -> 82, 3B 141 -> 122, 7B 379 -> 340; 300 tokens 7B 72 -> 75, 14B 73 -> 77) and K from 1,280 on (0.5B,
+//     whose products are too short for the epilogue, at 2,048 tokens 37 -> 44), and where the host is the bound: 300 tokens 0.5B 12 -> 14, 1.5B
+//     20 -> 21, 3B 32 -> 31; a 0.5B step of 300 tokens with all of these 3,120 -> 2,582 us queued, 1,181 -> 1,245 replayed.
+//   Modes 5 and 6, whose epilogues take longer: 47 % and K from 3,072 on (0.96 to 1.17 times as fast).  K 896 to 2,048 takes 0.66 to
+//     1.04: Peratar's 1.5B step of 505 tokens replayed 3,368 -> 3,831, queued 5,132 -> 4,749.
+static bool gw_pays(int mode, int T, int N, int K, bool chunked) {
+  const int width = mode == 2 ? N : K;
+  const bool narrow = width < 3072 && (long long)T * width <= 3 << 19;
+  if (mode == 2 && 2LL * K >= 5LL * N ? chunked && T <= GW_CHUNKED_TOKENS : (mode == 2 || mode == 3) && narrow) return true;
+  if (K < (mode == 2 ? 2048 : mode == 3 ? 1280 : 3072)) return false;
+  const long long rows = mode == 3 || mode == 6 ? 2LL * N : N;
+  const int pairs = gw_pairs();
+  int bn, chunks;
+  const double cycles = choose_tile(T, (int)((rows + 2 * UMMA_M - 1) / (2 * UMMA_M)), (K + GW_BK - 1) / GW_BK, pairs, 1, bn, chunks);
+  // (A pair makes 8,192 multiply-adds a cycle.)
+  return (double)rows * T * K >= (mode == 2 ? 0.49 : 0.47) * 8192.0 * pairs * cycles;
+}
 
 template <int MODE>
 static int launch_wide(const CUtensorMap& mw, const CUtensorMap& mx, const WideArgs& g, int pairs, cudaStream_t stream) {
@@ -487,6 +518,11 @@ static int gemm_bf16_wide(const void* x, int x_rows, const void* w, int mode, Wi
 using namespace vx;
 
 VX_TRACE_API(vx_wide)
+
+// 1 where a product of a long step is better off here than with a library (mode 2: chunked says whether K may be cut).
+VX_API int vx_gemm_bf16_wide_pays(int mode, int T, int N, int K, int chunked) {
+  return T > 0 && N > 0 && K > 0 && gw_pays(mode, T, N, K, chunked != 0) ? 1 : 0;
+}
 
 // x [x_rows >= T, K] bf16, w [N, K] bf16 (modes 3 and 6: [2 N, K]); see the head of the file for the modes.  tokens: of a
 // tile, chunks of K (mode 2): 0 for what takes least.  Return 0 on launch, a cudaError_t on failure, -1 for sizes and

@@ -60,6 +60,7 @@ def core():
         lib.vx_gemm_bf16_wide_glu.argtypes = [
             _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_ll, _c_int, _c_f, _c_f, _c_f, _c_f, _ptr, _ptr,
         ]
+        lib.vx_gemm_bf16_wide_pays.argtypes = [_c_int] * 5
         lib.vx_gemm_bf16_wide_xielu.argtypes = [
             _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_ll, _c_ll, _c_int, _c_int, _c_f, _c_f, _ptr, _ptr,
         ]
@@ -871,6 +872,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
 
 
 GEMM_OUT_BF16, GEMM_OUT_F32, GEMM_ADD_F32, GEMM_SWIGLU = 0, 1, 2, 3
+GEMM_XIELU, GEMM_GLU = 5, 6  # epilogues with wrappers of their own
 
 
 def gemm_bf16_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -916,6 +918,12 @@ def gemm_bf16(
             "multiple of 8 and both operands 16-byte aligned"
         )
     _check(code, "gemm_bf16")
+
+
+def gemm_bf16_wide_pays(mode: int, num_rows: int, out_features: int, in_features: int, chunked: bool) -> bool:
+    """Whether a product of a long step takes less on pairs of SMs than as a library product with the kernel that follows
+    it (gw_pays in gemm_bf16_wide.cu); ``out_features`` of a gated matrix are half its rows, ``chunked``: sums may cut the inner size."""
+    return core().vx_gemm_bf16_wide_pays(mode, num_rows, out_features, in_features, int(chunked)) != 0
 
 
 def gemm_bf16_wide(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, mode: int,

@@ -9,13 +9,14 @@ bfloat16: the tcgen05/TMA kernel of ``csrc/gemm_bf16.cu`` when the step has few 
 and short portions: the weight fills the 128-row side of the tensor-core tile and is streamed
 once; projections with few output tiles are split along K over a thread-block cluster); for long
 portions the one of ``csrc/gemm_bf16_wide.cu`` (pairs of SMs) where an activation or the sum into the
-stream follows in its epilogue, and a library GEMM (cuBLAS through torch) where nothing does and for
-inner sizes the TMA tiles cannot take.  The
-reference engine uses a library GEMM for every projection (``nn.Linear``,
+stream follows in its epilogue and this is the better way (``gw_pays`` there), and a library GEMM
+(cuBLAS through torch) for the others and for inner sizes the TMA tiles cannot take.  The reference
+engine uses a library GEMM for every projection (``nn.Linear``,
 src/self_attention.py:32-33, src/mlp.py:9-10, src/transformer.py:60 of that project).
 """
 from __future__ import annotations
 
+import functools
 import os
 from typing import Optional
 
@@ -45,8 +46,14 @@ def use_tensor_core_kernel(x, weight: torch.Tensor, num_rows: int) -> bool:
     )
 
 
-def use_wide_kernel(x, weight: torch.Tensor, num_rows: int, status) -> bool:
-    """Long steps: the kernel on pairs of SMs."""
+def use_wide_kernel(x, weight: torch.Tensor, num_rows: int, status, mode: int) -> bool:
+    """Long steps: whether a product with this epilogue (``GEMM_ADD_F32``, ``GEMM_SWIGLU``, ``GEMM_XIELU`` or
+    ``GEMM_GLU``) goes to the kernel on pairs of SMs."""
+    return (num_rows > SMALL_STEP_TOKENS and weight.dtype == torch.bfloat16
+            and _wide_pays(mode, num_rows, *weight.shape) and _wide_takes(x, weight, num_rows, status))
+
+
+def _wide_takes(x, weight: torch.Tensor, num_rows: int, status) -> bool:
     if _is_pending_norm(x):
         x = x.out
     return (
@@ -57,9 +64,16 @@ def use_wide_kernel(x, weight: torch.Tensor, num_rows: int, status) -> bool:
     )
 
 
+@functools.lru_cache(maxsize=4096)
+def _wide_pays(mode: int, num_rows: int, rows: int, in_features: int) -> bool:
+    gated = mode in (kernels.GEMM_SWIGLU, kernels.GEMM_GLU)
+    return kernels.gemm_bf16_wide_pays(mode, num_rows, rows // 2 if gated else rows, in_features, _CHUNKED_SPLITK)
+
+
 def adds_to_stream(x, weight: torch.Tensor, num_rows: int, status) -> bool:
-    """Whether ``linear`` can add this product into float32 rows (``accumulate``)."""
-    return status is not None and (use_tensor_core_kernel(x, weight, num_rows) or use_wide_kernel(x, weight, num_rows, status))
+    """Whether this product is to be added into float32 rows by ``linear`` (``accumulate``)."""
+    return status is not None and (use_tensor_core_kernel(x, weight, num_rows)
+                                   or use_wide_kernel(x, weight, num_rows, status, kernels.GEMM_ADD_F32))
 
 
 def _is_pending_norm(x) -> bool:
@@ -94,10 +108,11 @@ def choose_splits(out_features: int, in_features: int, num_rows: int = 1, tile: 
 
 
 # VELOX_B200_NO_CHUNKED_SPLITK=1 keeps the sums into the residual stream in a fixed order (the
-# cluster form of split K), for bisecting.  VELOX_B200_DETERMINISTIC=1 does that and keeps the
-# feed-forward of small steps as two kernels: every sum of the bfloat16 path then has a fixed
-# order and a run repeats bit by bit (seeded sampling gives the same tokens again), at the
-# price of the two fastest forms of small steps.
+# cluster form of split K; one chunk or the library in steps of 257 to 768 tokens, beyond which no sum is cut), for
+# bisecting.  VELOX_B200_DETERMINISTIC=1 does that and keeps the feed-forward of small steps as two
+# kernels: every sum of the bfloat16 path then has a fixed order and a run repeats bit by bit (seeded
+# sampling gives the same tokens again), at the price of the two fastest forms of small steps and of the
+# down projection's in those of 257 to 768 tokens.
 DETERMINISTIC = os.environ.get("VELOX_B200_DETERMINISTIC") == "1"
 _CHUNKED_SPLITK = os.environ.get("VELOX_B200_NO_CHUNKED_SPLITK") != "1" and not DETERMINISTIC
 
@@ -177,7 +192,7 @@ def linear(
         kernels.gemm_bf16(x, weight, bias_f32, out, mode, num_rows, status,
                           splits=choose_splits(weight.shape[0], weight.shape[1], num_rows))
         return out
-    if accumulate and scale is None and mirror is None and use_wide_kernel(x, weight, num_rows, status):
+    if accumulate and scale is None and mirror is None and _wide_takes(x, weight, num_rows, status):
         if kernels.gemm_bf16_wide(x, weight, bias_f32, out, kernels.GEMM_ADD_F32, num_rows, status,
                                   chunks=0 if _CHUNKED_SPLITK else 1):
             return out
@@ -218,12 +233,11 @@ def swiglu_linear(
     status: torch.Tensor,
 ) -> torch.Tensor:
     """out = silu(x @ Wg.T) * (x @ Wu.T) in one kernel (gate and up rows of one matrix)."""
-    if use_wide_kernel(x, gate_up_weight, num_rows, status):
+    if _wide_takes(x, gate_up_weight, num_rows, status):
         if _is_pending_norm(x):
             x = x.materialize()
-        if not kernels.gemm_bf16_wide(x, gate_up_weight, None, out, kernels.GEMM_SWIGLU, num_rows, status):
-            raise kernels.KernelError(f"gemm_bf16_wide refuses w {tuple(gate_up_weight.shape)}")
-        return out
+        if kernels.gemm_bf16_wide(x, gate_up_weight, None, out, kernels.GEMM_SWIGLU, num_rows, status):
+            return out
     if _is_pending_norm(x):
         if _fuses_norm(x, gate_up_weight, num_rows, status):
             if kernels.gemm_bf16_normed(x.resid, x.weight, x.eps, gate_up_weight, None, out,

@@ -255,7 +255,7 @@ class LatentAttention(Mixer):
         """W_o: straight into the stream the block offers (bfloat16), or a product of its own."""
         if (ctx.residual is not None and ctx.status is not None and self.dtype != torch.float32
                 and (use_tensor_core_kernel(heads_out, self.w_out, T)
-                     or (ctx.residual_scale is None and use_wide_kernel(heads_out, self.w_out, T, ctx.status)))):
+                     or (ctx.residual_scale is None and use_wide_kernel(heads_out, self.w_out, T, ctx.status, kernels.GEMM_ADD_F32)))):
             linear(heads_out, self.w_out, None, ctx.residual, T, status=ctx.status, accumulate=True,
                    scale=ctx.residual_scale)
             return None

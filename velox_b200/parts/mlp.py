@@ -57,21 +57,21 @@ class SwiGLU(FeedForward):
             if kernels.mlp_fused(x.resid, x.weight, x.eps, self.w_gate_up, self.w_down, ctx.residual, T, ctx.status):
                 return None
         act = ws.get("swiglu.act", (ws.max_tokens, self.intermediate_size), self.dtype)
-        if adds_to_stream(x, self.w_gate_up, T, ctx.status) and adds_to_stream(act, self.w_down, T, ctx.status):
-            # SiLU(gate) * up in the projection's epilogue, then the down projection added straight
-            # into the float32 residual stream.
+        if use_wide_kernel(x, self.w_gate_up, T, ctx.status, kernels.GEMM_SWIGLU) or (
+                ctx.status is not None and use_tensor_core_kernel(x, self.w_gate_up, T)
+                and use_tensor_core_kernel(act, self.w_down, T)):
+            # SiLU(gate) * up in the projection's epilogue.
             swiglu_linear(x, self.w_gate_up, act, T, ctx.status)
-            if ctx.residual is not None:
-                linear(act, self.w_down, None, ctx.residual, T, status=ctx.status, accumulate=True)
-                return None
-            out = ws.get("feed_forward.out", (ws.max_tokens, self.hidden_size), self.dtype)
-            linear(act, self.w_down, None, out, T, status=ctx.status)
-            return out
-        gate_up = ws.get("swiglu.gate_up", (ws.max_tokens, 2 * self.intermediate_size), self.dtype)
-        linear(x, self.w_gate_up, None, gate_up, T)
-        kernels.swiglu(gate_up, act, T)
+        else:
+            gate_up = ws.get("swiglu.gate_up", (ws.max_tokens, 2 * self.intermediate_size), self.dtype)
+            linear(x, self.w_gate_up, None, gate_up, T, status=ctx.status)
+            kernels.swiglu(gate_up, act, T)
+        if ctx.residual is not None and adds_to_stream(act, self.w_down, T, ctx.status):
+            # The down projection goes straight into the float32 residual stream.
+            linear(act, self.w_down, None, ctx.residual, T, status=ctx.status, accumulate=True)
+            return None
         out = ws.get("feed_forward.out", (ws.max_tokens, self.hidden_size), self.dtype)
-        linear(act, self.w_down, None, out, T)
+        linear(act, self.w_down, None, out, T, status=ctx.status)
         return out
 
 
@@ -125,7 +125,7 @@ class DenseXielu(FeedForward):
                  and kernels.gemm_bf16_xielu(x, self.w_up[: self.side_rows + self.intermediate_size],
                                              self.b_up, up, act, self.side_rows, self.a_pos, self.a_neg, T,
                                              ctx.status, splits=choose_splits(self.up_width, self.hidden_size, T)))
-        if not fused and use_wide_kernel(x, self.w_up, T, ctx.status):
+        if not fused and use_wide_kernel(x, self.w_up, T, ctx.status, kernels.GEMM_XIELU):
             fused = kernels.gemm_bf16_wide_xielu(x, self.w_up[: self.side_rows + self.intermediate_size], self.b_up, up, act,
                                                  self.side_rows, self.a_pos, self.a_neg, T, ctx.status)
         if not fused:
@@ -274,7 +274,7 @@ class ClampedGLU(FeedForward):
             # Few tokens: biases, clamps and activation in the projection's epilogue.
             kernels.gemm_bf16_glu(x, self.w_gate_up, self.b_gate_up, act, T, self.limit, self.alpha, self.up_shift,
                                   ctx.status, cubic=self.cubic)
-        elif use_wide_kernel(x, self.w_gate_up, T, ctx.status) and kernels.gemm_bf16_wide_glu(
+        elif use_wide_kernel(x, self.w_gate_up, T, ctx.status, kernels.GEMM_GLU) and kernels.gemm_bf16_wide_glu(
                 x, self.w_gate_up, self.b_gate_up, act, T, self.limit, self.alpha, self.up_shift, ctx.status, cubic=self.cubic):
             pass  # the same for a long step
         else:
@@ -287,7 +287,7 @@ class ClampedGLU(FeedForward):
         ws = ctx.workspace
         if (ctx.residual is not None and ctx.status is not None and self.dtype != torch.float32
                 and (use_tensor_core_kernel(act, self.w_down, T)
-                     or (ctx.residual_scale is None and use_wide_kernel(act, self.w_down, T, ctx.status)))):
+                     or (ctx.residual_scale is None and use_wide_kernel(act, self.w_down, T, ctx.status, kernels.GEMM_ADD_F32)))):
             # The down projection (and its bias) goes straight into the float32 stream.
             linear(act, self.w_down, self.b_down, ctx.residual, T, status=ctx.status, accumulate=True,
                    scale=ctx.residual_scale)
