@@ -233,7 +233,7 @@ def swiglu_linear(
     status: torch.Tensor,
 ) -> torch.Tensor:
     """out = silu(x @ Wg.T) * (x @ Wu.T) in one kernel (gate and up rows of one matrix)."""
-    if _wide_takes(x, gate_up_weight, num_rows, status):
+    if num_rows > SMALL_STEP_TOKENS and _wide_takes(x, gate_up_weight, num_rows, status):
         if _is_pending_norm(x):
             x = x.materialize()
         if kernels.gemm_bf16_wide(x, gate_up_weight, None, out, kernels.GEMM_SWIGLU, num_rows, status):

@@ -10,8 +10,7 @@ import os
 import torch
 
 from ..ops import kernels
-from ..ops.linear import (DETERMINISTIC, adds_to_stream, choose_splits, linear, swiglu_linear, use_tensor_core_kernel,
-                          use_wide_kernel)
+from ..ops.linear import DETERMINISTIC, choose_splits, linear, swiglu_linear, use_tensor_core_kernel, use_wide_kernel
 from .base import FeedForward, PendingSums
 from .registry import register_part
 
@@ -57,16 +56,16 @@ class SwiGLU(FeedForward):
             if kernels.mlp_fused(x.resid, x.weight, x.eps, self.w_gate_up, self.w_down, ctx.residual, T, ctx.status):
                 return None
         act = ws.get("swiglu.act", (ws.max_tokens, self.intermediate_size), self.dtype)
-        if use_wide_kernel(x, self.w_gate_up, T, ctx.status, kernels.GEMM_SWIGLU) or (
-                ctx.status is not None and use_tensor_core_kernel(x, self.w_gate_up, T)
-                and use_tensor_core_kernel(act, self.w_down, T)):
+        adds = ctx.status is not None and use_tensor_core_kernel(act, self.w_down, T)
+        if (adds and use_tensor_core_kernel(x, self.w_gate_up, T)
+                or use_wide_kernel(x, self.w_gate_up, T, ctx.status, kernels.GEMM_SWIGLU)):
             # SiLU(gate) * up in the projection's epilogue.
             swiglu_linear(x, self.w_gate_up, act, T, ctx.status)
         else:
             gate_up = ws.get("swiglu.gate_up", (ws.max_tokens, 2 * self.intermediate_size), self.dtype)
             linear(x, self.w_gate_up, None, gate_up, T, status=ctx.status)
             kernels.swiglu(gate_up, act, T)
-        if ctx.residual is not None and adds_to_stream(act, self.w_down, T, ctx.status):
+        if ctx.residual is not None and (adds or use_wide_kernel(act, self.w_down, T, ctx.status, kernels.GEMM_ADD_F32)):
             # The down projection goes straight into the float32 residual stream.
             linear(act, self.w_down, None, ctx.residual, T, status=ctx.status, accumulate=True)
             return None
