@@ -70,7 +70,7 @@ class LinearHead(Part):
         ws = ctx.workspace
         logits = ws.get("lm_head.logits", (ws.max_logit_rows, self.vocab_size), torch.float32)
         if self.dtype == torch.float32:
-            linear(x, self.weight, None, logits, num_rows)
+            linear(x, self.weight, None, logits, num_rows, status=ctx.status)
         elif use_tensor_core_kernel(x, self.weight, num_rows):
             # float32 logits straight from the accumulators
             linear(x, self.weight, None, logits, num_rows, status=ctx.status)
