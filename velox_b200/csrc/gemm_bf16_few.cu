@@ -12,7 +12,7 @@
 // in gemm_bf16.cu.  The order of a sum is fixed.
 //
 // Modes (as in gemm_bf16.cu): 0 bf16 + bias, 1 float32 + bias, 2 float32 += (and a copy of the sums), 4 q | k | v of
-// whole heads with rotation and cache write: a tile is eight pairs (d, d + half a head).
+// whole heads with rotation and cache write: a tile is eight pairs (d, d + half a head).  With the norm inside: 4 only.
 #include "common.cuh"
 #include "gemm_bf16_few.cuh"
 
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_bf16_few_kernel(const FewArgs
   // What the output adds to is asked for with the input.
   constexpr int OUTPUTS = (FEW_ROWS * 8 * TILES + WARPS * 32 - 1) / (WARPS * 32);
   float old[OUTPUTS];
-  if (g.mode == 2) {
+  if (!NORM && g.mode == 2) {
 #pragma unroll
     for (int u = 0; u < OUTPUTS; ++u) {
       const int e = threadIdx.x + u * WARPS * 32, t = e / FEW_ROWS, r = e % FEW_ROWS;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_bf16_few_kernel(const FewArgs
     }
     return g.bias != nullptr ? v + g.bias[n] : v;
   };
-  if (g.mode == 4) {
+  if (NORM || g.mode == 4) {
     const int half = apart, head = first / g.head_dim;
     const bool is_q = head < g.heads, is_k = !is_q && head < g.heads + g.kv_heads;
     for (int e = threadIdx.x; e < 8 * g.T; e += WARPS * 32) {
@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_bf16_few_kernel(const FewArgs
 // the weights no longer come at once (12.0 | 7.6 -> 13.4 | 8.8).
 bool gemm_bf16_few_takes(int T, int N, int K, int mode, bool norm) {
   if (T > 16 || (mode != 0 && mode != 1 && mode != 2 && mode != 4) || (N + FEW_ROWS - 1) / FEW_ROWS > 2 * 148) return false;
-  // (Plain outputs with the norm inside keep the ring kernel and its order of sums: no step that was timed makes them, and of a
-  // small model's 53 rows in bfloat16, of which one may miss its tolerance against separate requests, two did with this one's.)
+  // (Plain outputs with the norm inside stay with the ring kernel, where they were before this one was there.  Here they would be
+  // as near to 64 bits, 7e-8 to 1.2e-7 in the 2-norm beside the operands' rounding where the ring has 8e-8 to 7.6e-7, and sooner: one
+  // token by 64 x 128 1.3 us against 4.8, 1,152 x 896 2.8 against 7.6, 2,048 x 1,536 4.8 against 9.2.  Open.)
   if (norm && mode != 4) return false;
   return K <= (T > 8 ? 1024 : norm ? 1536 : 2048);
 }
