@@ -30,8 +30,7 @@ KERNEL_NAMES = {
     1: "embed", 2: "norm", 3: "rope/swiglu", 10: "gemm bf16 out", 11: "gemm f32 out", 12: "gemm += stream",
     13: "gemm swiglu", 14: "gemm qkv+rope", 15: "mlp one kernel", 20: "attn mma.sync", 21: "attn narrow",
     22: "attn merge", 23: "attn tcgen05", 30: "gemm few bf16 out", 31: "gemm few f32 out", 32: "gemm few += stream",
-    34: "gemm few qkv+rope", 40: "gemm wide bf16 out", 42: "gemm wide += stream", 43: "gemm wide swiglu",
-    44: "gemm wide qkv+rope", 45: "gemm wide xielu", 46: "gemm wide glu",
+    34: "gemm few qkv+rope", 42: "gemm wide += stream", 43: "gemm wide swiglu", 45: "gemm wide xielu", 46: "gemm wide glu",
 }
 TC_ATTENTION = 23
 EVENT_BYTES = 64

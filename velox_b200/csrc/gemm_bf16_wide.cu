@@ -350,19 +350,19 @@ gemm_bf16_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 // ---------------------------------------------------------------------------------------------
 // Host side.
 // ---------------------------------------------------------------------------------------------
-// A bf16 matrix [rows, K] as a map of up to four dimensions, the innermost along K in boxes of 64: extents, pitches (in
-// elements) and box extents of the others.
+// A bf16 matrix as a map whose innermost dimension runs along K in boxes of 64: extents, pitches (in elements) and box
+// extents of the one or two others.
 struct WideMap {
   int dims;
-  long long extent[3], pitch[3];
-  int box[3];
+  long long extent[2], pitch[2];
+  int box[2];
 };
 
 static bool gw_tensor_map(CUtensorMap* map, const void* base, long long K, const WideMap& m) {
-  using Key = std::tuple<const void*, long long, long long, long long, long long, int, int, int>;
+  using Key = std::tuple<const void*, long long, int, long long, long long, int, int>;
   static std::map<Key, CUtensorMap> cache;
   static std::mutex lock;
-  const Key key{base, K, m.extent[0], m.extent[1], m.extent[2], m.box[0], m.box[1], m.box[2] * 8 + m.dims};
+  const Key key{base, K, m.dims, m.extent[0], m.extent[1], m.box[0], m.box[1]};  // (the pitches follow from these)
   std::lock_guard<std::mutex> guard(lock);
   const auto it = cache.find(key);
   if (it != cache.end()) {
@@ -371,8 +371,8 @@ static bool gw_tensor_map(CUtensorMap* map, const void* base, long long K, const
   }
   const EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return false;
-  cuuint64_t extent[4] = {(cuuint64_t)K}, pitch[3];
-  cuuint32_t box[4] = {GW_BK}, step[4] = {1, 1, 1, 1};
+  cuuint64_t extent[3] = {(cuuint64_t)K}, pitch[2];
+  cuuint32_t box[3] = {GW_BK}, step[3] = {1, 1, 1};
   for (int i = 0; i < m.dims; ++i) {
     extent[i + 1] = (cuuint64_t)m.extent[i];
     pitch[i] = (cuuint64_t)m.pitch[i] * 2;
@@ -500,10 +500,10 @@ static int gemm_bf16_wide(const void* x, int x_rows, const void* w, int mode, Wi
   if ((long long)weight_tiles * g.token_tiles * g.chunks > 1 << 30) return -1;
   g.tiles = weight_tiles * g.token_tiles;
   CUtensorMap mw, mx;
-  WideMap wide = {1, {N, 1, 1}, {K, 0, 0}, {UMMA_M, 1, 1}};
-  if (gated) wide = {2, {2, N, 1}, {(long long)N * K, K, 0}, {2, UMMA_M / 2, 1}};
+  WideMap wide = {1, {N, 1}, {K, 0}, {UMMA_M, 1}};
+  if (gated) wide = {2, {2, N}, {(long long)N * K, K}, {2, UMMA_M / 2}};
   if (!gw_tensor_map(&mw, w, K, wide)) return -1;
-  if (!gw_tensor_map(&mx, x, K, WideMap{1, {x_rows, 1, 1}, {K, 0, 0}, {g.bn / 2, 1, 1}})) return -1;
+  if (!gw_tensor_map(&mx, x, K, WideMap{1, {x_rows, 1}, {K, 0}, {g.bn / 2, 1}})) return -1;
   switch (mode) {
     case 2: return launch_wide<2>(mw, mx, g, pairs, stream);
     case 3: return launch_wide<3>(mw, mx, g, pairs, stream);
