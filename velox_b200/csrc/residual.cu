@@ -264,7 +264,8 @@ __global__ void cast_rows_kernel(const float* __restrict__ in, __nv_bfloat16* __
 // load needs (16 bytes in float32, 8 in bfloat16): a thread keeps up to GV_CHUNKS chunks in
 // registers across the two reductions: four warps a row and up to four chunks a thread (rows of
 // up to 2,048 elements), or eight warps and up to eight chunks (up to 8,192).  The same formulas;
-// the order of a row's sums depends on the row's length only.
+// the order of a row's sums depends on the row's length only in float32.  bfloat16 rows of up to 4,096
+// elements in launches of up to GV_FEW_ROWS rows have one chunk a thread, and another order with it.
 // ---------------------------------------------------------------------------------------------
 constexpr int GV_CHUNKS = 8;
 constexpr int GV_FEW_ROWS = 148;  // a row an SM
