@@ -453,7 +453,7 @@ def run_own(args):
             "vocab": cfg["vocab_size"], "global_batch": args.batch, "seq_len": CONTEXT, "prefill_tokens": PREFILL_TOKENS,
             "kv_block_size": block_size, "kv_block_size_engine_default": ENGINE_DEFAULT_BLOCK_SIZE, "tied_embeddings": True, "parallelism": "single GPU",
             "l2": "inputs larger than L2 (weights streamed every step)",
-            "decode_steps": "queued back to back; each is fed the tokens the step before sampled, on the device; 40 more untimed steps before the timed ones", "gemm": "decode: own kernels (tcgen05; mma.sync for small projections of a few tokens); prefill: own, QKV cuBLAS (library)",
+            "decode_steps": "queued back to back; each is fed the tokens the step before sampled, on the device; 40 more untimed steps before the timed ones", "gemm": "decode: own kernels (tcgen05; mma.sync for small projections of a few tokens); prefill: own tcgen05 kernels where an epilogue follows and pays, else cuBLAS (library)",
         },
         "clocks": clock_summary,
         "e2e": e2e,

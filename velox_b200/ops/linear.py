@@ -1,7 +1,8 @@
 """Matrix products of the model: ``y = x @ W.T + b`` with W stored [out, in].
 
 float32: this package's own GEMM, always (no TF32, no library): small matrices on the FP32 pipes, large ones on the
-tensor cores as products of three-term bfloat16 splits with float32 sums, nearer the exact sums than a chain of FMAs.
+tensor cores as products of three-term bfloat16 splits with float32 sums, nearer the exact sums than a chain of FMAs
+unless one or two products carry a sum.
 Which of the two follows from the matrix alone (rows that do not begin at multiples of 16 bytes stay on the
 FP32 pipes), and every output element is summed in a fixed order.
 
