@@ -165,3 +165,46 @@ def test_feed_forward_on_both_sides_of_the_lines(k, status, T, E, I, gate, down)
     assert (got[:T].double() - want).abs().max().item() <= bound
     assert torch.equal(stream[T:], start[T:]) and (down or torch.equal(stream, start))
     assert int(status[0]) == 0
+
+
+def test_long_steps_repeat_with_the_switch():
+    """VELOX_B200_DETERMINISTIC=1 (read at import, hence a process of its own): no sum of a long step is cut, also where
+    the default cuts it (down projections of up to 768 tokens)."""
+    import os
+    import pathlib
+    import subprocess
+    import sys
+
+    program = """
+from types import SimpleNamespace
+import torch
+from velox_b200.engine.runner import Workspace
+from velox_b200.ops.linear import adds_to_stream, linear
+from velox_b200.parts.mlp import SwiGLU
+dev = torch.device("cuda")
+E, I = 1536, 8960
+gen = torch.Generator(device=dev).manual_seed(1)
+def matrix(rows, cols):
+    return (torch.randn(rows, cols, generator=gen, device=dev) / cols ** 0.5).to(torch.bfloat16)
+part = SwiGLU({"hidden_size": E, "intermediate_size": I}, {"gate_up.weight": matrix(2 * I, E), "down.weight": matrix(E, I)},
+              torch.bfloat16, dev)
+w_out = matrix(E, E)
+status = torch.zeros(4, dtype=torch.int32, device=dev)
+for T in (257, 700, 1030):
+    x, act = matrix(T, E), matrix(T, I)
+    assert not (T < 768 and adds_to_stream(act, part.w_down, T, status))
+    first = None
+    for _ in range(6):
+        stream = torch.ones(T, E, device=dev)
+        linear(x, w_out, None, stream, T, status=status, accumulate=True)
+        linear(act, part.w_down, None, stream, T, status=status, accumulate=True)
+        out = part.forward(x, SimpleNamespace(num_tokens=T, workspace=Workspace(T, 8, dev), residual=stream, status=status))
+        both = [stream] + ([] if out is None else [out[:T].clone()])
+        first = both if first is None else first
+        assert all(torch.equal(a, b) for a, b in zip(both, first)), T
+assert int(status[0]) == 0
+"""
+    root = str(pathlib.Path(__file__).resolve().parent.parent)
+    env = dict(os.environ, VELOX_B200_DETERMINISTIC="1", PYTHONPATH=root + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    done = subprocess.run([sys.executable, "-c", program], env=env, cwd=root, capture_output=True, text=True, timeout=240)
+    assert done.returncode == 0, done.stderr[-2000:]
